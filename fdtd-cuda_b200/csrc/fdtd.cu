@@ -17,6 +17,7 @@
 #include "../../include/fdtd_b200.h"
 #include "kernels.cuh"
 #include "staged.cuh"
+#include "flat.cuh"
 #include "boundary.cuh"
 #include "adjoint.cuh"
 #include "snapshot.cuh"
@@ -77,7 +78,9 @@ struct fdtd_sim {
   // (interior tiles: minb/stages, CPML edge tiles: eminb/estages)
   // pdl = 1: the edge and interior launches of a pass go on one stream
   // with a programmatic dependency instead of on two streams
-  struct PassCfg { int minb = 1, ty = 4, kchunk = 16, staged = 1, stages = 4, eminb = 1, estages = 4, pdl = 0, tma = 0, etma = 0; float ms = 0; };
+  struct PassCfg { int minb = 1, ty = 4, kchunk = 16, staged = 1, stages = 4, eminb = 1, estages = 4, pdl = 0, tma = 0, etma = 0; float ms = 0;
+    // direct pass (flat.cuh): planes per thread and unrolled planes; kz = 0 = the staged pass
+    int kz = 0, unroll = 1; };
   // pass tiles for one (tile height, z-chunk): the interior box of tiles
   // that touch no CPML slab and the table of the others
   struct TileSet {
@@ -335,7 +338,7 @@ static fdtd_status build_views(fdtd_sim* s) {
     const CpmlTables& t = su.cp[a];
     const int Nc = su.Nc[a];
     T* base;
-    const size_t need = 8 * (size_t)(Nc + 1) + (size_t)(Nc + 1) + 2 * (size_t)N3[a];
+    const size_t need = 9 * (size_t)(Nc + 1) + 7 * ((size_t)N3[a] + 16);
     cudaError_t e = s->alloc(&base, need);
     if (e != cudaSuccess) return fail(FDTD_ERR_ALLOC, cudaGetErrorString(e));
     T* q = base;
@@ -355,11 +358,37 @@ static fdtd_status build_views(fdtd_sim* s) {
     ca.ch_N = put(t.ch_N, Nc + 1); ca.ch_F = put(t.ch_F, Nc + 1);
     std::vector<double> ik(N3[a]), ih(N3[a]);
     for (int i = 0; i < N3[a]; i++) { ik[i] = 1.0 / t.ked[i]; ih[i] = 1.0 / t.khd[i]; }
-    ca.inv_ked = put(ik, N3[a]);
-    ca.inv_khd = put(ih, N3[a]);
+    // tables over the whole axis: 16-byte aligned, padded to the row pitch
+    const size_t full = ((size_t)N3[a] + 7) / 8 * 8;
+    auto align = [&]() { q += (8 - (q - base) % 8) % 8; };
+    align();
+    ca.inv_ked = put(ik, full);
+    ca.inv_khd = put(ih, full);
     ca.inv_d = (T)(1.0 / dxyz[a]);
     ca.Nc = Nc;
     ca.F = su.F[a];
+    auto whole = [&](const std::vector<double>& near_, const std::vector<double>& far_) {
+      std::vector<double> v(full, 0.0);
+      for (int i = 0; i < (int)near_.size() && i < N3[a]; i++) v[i] = near_[i];
+      for (int i = 0; i < (int)far_.size() && su.F[a] + i < N3[a]; i++) v[su.F[a] + i] = far_[i];
+      return v;
+    };
+    // the near slab reads the first Nc+1 entries of the source table
+    auto first = [&](std::vector<double> src) {
+      src.resize(std::max(Nc + 1, 0), 0.0);
+      return src;
+    };
+    ca.be = put(whole(t.be_N, t.be_F), full);
+    ca.ce = put(whole(t.ce_N, t.ce_F), full);
+    ca.bh = put(whole(t.bh_N, t.bh_F), full);
+    ca.ch = put(whole(t.ch_N, t.ch_F), full);
+    ca.ce_ey = ca.ce;
+    if (a == 0)
+      ca.ce_ey = put(whole(first((su.p.fixes & FDTD_FIX_CE_EY_XN) ? su.cp[0].ce_N : su.cp[1].ce_N), t.ce_F), full);
+    constexpr int V = Vec<T>::N;
+    ca.Wn = (std::max(Nc, 0) + 1 + V - 1) / V * V;
+    ca.fb = std::min(s->PX, std::max(su.F[a] / V * V, ca.Wn));
+    ca.W = ca.Wn + (a == 0 ? s->PX - ca.fb : 0);
     v.dxyz[a] = (T)dxyz[a];
     // Ey's near-x slab reads ce_y_N in the reference (main.cu:2891)
     if (a == 0) {
@@ -382,15 +411,17 @@ static fdtd_status build_views(fdtd_sim* s) {
       size_t cells_e, cells_h;
       if (ax == 2) { cells_e = (size_t)(Nc + 1) * s->plane; cells_h = (size_t)Nc * s->plane; }
       else if (ax == 1) { cells_e = (size_t)s->NZ * (Nc + 1) * s->PX; cells_h = (size_t)s->NZ * Nc * s->PX; }
-      else { cells_e = (size_t)s->NZ * s->NY * (Nc + 1); cells_h = (size_t)s->NZ * s->NY * Nc; }
+      else { cells_e = cells_h = (size_t)s->NZ * s->NY * v.cp[0].W; }
       // near slab then far slab in one allocation (the passes index both
       // from the near pointer)
       T *a1, *a3;
       cudaError_t e;
-      if ((e = s->alloc(&a1, 2 * cells_e, true)) != cudaSuccess || (e = s->alloc(&a3, 2 * cells_h, true)) != cudaSuccess)
+      // (the x axis's rows hold both slabs)
+      const int both = ax == 0 ? 1 : 2;
+      if ((e = s->alloc(&a1, both * cells_e, true)) != cudaSuccess || (e = s->alloc(&a3, both * cells_h, true)) != cudaSuccess)
         return fail(FDTD_ERR_ALLOC, cudaGetErrorString(e));
-      v.psiE_N[c][slot] = a1; v.psiE_F[c][slot] = a1 + cells_e;
-      v.psiH_N[c][slot] = a3; v.psiH_F[c][slot] = a3 + cells_h;
+      v.psiE_N[c][slot] = a1; v.psiE_F[c][slot] = a1 + (ax == 0 ? (size_t)v.cp[0].Wn : cells_e);
+      v.psiH_N[c][slot] = a3; v.psiH_F[c][slot] = a3 + (ax == 0 ? (size_t)v.cp[0].Wn : cells_h);
     }
   // TFSF
   TfsfView& tf = v.tf;
@@ -941,7 +972,6 @@ static void staged_attributes() {
                        (int)staged_smem<T, TY, S>());
   FDTD_STAGED_VARIANTS(FDTD_ATTR)
 #undef FDTD_ATTR
-  cudaFuncSetAttribute(dft_contract<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_smem_bytes<T>());
   done = true;
 }
 
@@ -1033,6 +1063,40 @@ static void launch_e_variant(fdtd_sim* s, int ty, int mb, int sg, bool tma, dim3
   launch_variant<T, PML, true>(s, ty, mb, sg, tma, g, tm, kchunk, st, pdl);
 }
 
+// A launch on `st` that, when pdl is set, carries a programmatic dependency
+// on the launch before it on the stream: it may start once every CTA of
+// that launch has started, and orders itself with griddepcontrol.wait.
+template <typename... P, typename... A>
+static void launch_ex(bool pdl, void (*kern)(P...), dim3 g, dim3 blk, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = blk;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+// One launch of a direct pass (flat.cuh): kz planes per thread, one block per
+// kFlatThreads vectors and kz planes.  The H pass has a form whose plane loop
+// is unrolled by 8 (H reads E of plane k + 1, so the next plane's loads only
+// start early when the unrolled body hoists them: 256^3 FP32 119.7 us against
+// 136.8 rolled at kz = 8, 384 x 384 x 256 253.6 against 288.4); the E pass
+// reads plane k - 1, carried in registers, and is faster rolled (124.3 us
+// against 177.2).
+template <typename T, bool EPASS>
+static void launch_flat(fdtd_sim* s, int kz, int unroll, cudaStream_t st, bool pdl) {
+  const unsigned nv = (unsigned)(s->plane / Vec<T>::N), nbx = (nv + kFlatThreads - 1) / kFlatThreads;
+  const dim3 g(nbx * (unsigned)((s->NZ + kz - 1) / kz)), blk(kFlatThreads);
+  if (EPASS) launch_ex(pdl, e_flat<T, 1>, g, blk, 0, st, view<T>(s), nbx, kz);
+  else if (unroll == 8) launch_ex(pdl, h_flat<T, 8>, g, blk, 0, st, view<T>(s), nbx, kz);
+  else launch_ex(pdl, h_flat<T, 1>, g, blk, 0, st, view<T>(s), nbx, kz);
+}
+
 // Launches one pass as its interior box (PML-free) and its edge table so
 // that the two overlap: the edge launch on the side stream, or (c.pdl) the
 // edge launch then the interior launch with a programmatic dependency on
@@ -1042,6 +1106,10 @@ static void launch_e_variant(fdtd_sim* s, int ty, int mb, int sg, bool tma, dim3
 // first launch carries a programmatic dependency on it too.
 template <typename T, bool EPASS>
 static int launch_pass_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st, bool chained = false) {
+  if (c.kz) {
+    launch_flat<T, EPASS>(s, c.kz, c.unroll, st, chained);
+    return 1;
+  }
   const fdtd_sim::TileSet& ts = tiles(s, c);
   if (c.pdl && ((ts.inner.x && ts.nedge) || chained)) {
     bool dep = chained;
@@ -1086,12 +1154,94 @@ static int launch_e_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st
   return launch_pass_cfg<T, true>(s, c, st, chained);
 }
 
-// Autotuner: times every launch shape of the E and H passes on the zero
+// Autotuner of the staged passes: times every launch shape of the E and H passes on the zero
 // state (which they leave at zero: no source has run yet) and keeps the
 // fastest.  Shapes: minimum CTAs per SM (register cap) x tile height x
 // z-chunk.  FDTD_TUNE=0 keeps the defaults.
+
+// The direct passes: planes per thread of each pass.  More planes per thread
+// re-read less (the k +- 1 plane is carried) but leave fewer blocks, so small
+// grids want few and wave quantisation decides in between (96^3: 3 planes 8.3
+// us, 2 or 4 planes 10.3 us; 256^3: 8 planes): timed on the zero state like the
+// staged shapes.  Untimed (FDTD_TUNE=0, batch members, under 2^18 cells) the
+// most planes, up to 8, that leave two blocks a multiprocessor.
+// FDTD_PASS=flat:KZ[:UNROLL] fixes them.
+template <typename T>
+static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force) {
+  fdtd_sim::PassCfg def;
+  def.staged = 0;
+  def.pdl = 1;
+  const long long nbx = ((long long)(s->plane / Vec<T>::N) + kFlatThreads - 1) / kFlatThreads;
+  int sms = 148;
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  def.kz = 1;
+  while (def.kz < 8 && nbx * ((s->NZ + 2 * def.kz - 1) / (2 * def.kz)) >= 2 * sms) def.kz *= 2;
+  def.unroll = def.kz == 8 ? 8 : 1;
+  if (force) {
+    if (std::sscanf(force, "flat:%d:%d", &def.kz, &def.unroll) < 1 || def.kz < 1 ||
+        (def.unroll != 1 && def.unroll != 8))
+      return fail(FDTD_ERR_INVALID, "FDTD_PASS names a pass variant that is not built");
+  }
+  def.kchunk = def.kz;
+  def.stages = def.estages = def.unroll;
+  s->hcfg = s->ecfg = def;
+  s->tuned = true;
+  const char* env = std::getenv("FDTD_TUNE");
+  if (!time_variants || (env && env[0] == '0') || force || s->ncell < (size_t)(1 << 18)) return FDTD_OK;
+  const char* venv = std::getenv("FDTD_TUNE_VERBOSE");
+  const bool verbose = venv && venv[0] == '1';
+  cudaEvent_t a, b;
+  CUDA_TRY(cudaEventCreate(&a));
+  CUDA_TRY(cudaEventCreate(&b));
+  for (int pass = 0; pass < 2; pass++) {
+    fdtd_sim::PassCfg& best = pass == 0 ? s->hcfg : s->ecfg;
+    float best_ms = 1e30f;
+    for (int kz : {1, 2, 3, 4, 6, 8, 12, 16}) {
+      if (kz > s->NZ) continue;
+      for (int unroll : {1, 8}) {
+        if (unroll == 8 && (pass == 1 || kz < 8)) continue;
+        fdtd_sim::PassCfg c = def;
+        c.kz = c.kchunk = kz;
+        c.unroll = c.stages = c.estages = unroll;
+        auto go = [&]() {
+          if (pass == 0) launch_flat<T, false>(s, kz, unroll, 0, false);
+          else launch_flat<T, true>(s, kz, unroll, 0, false);
+        };
+        go();
+        go();
+        CUDA_TRY(cudaEventRecord(a));
+        for (int r = 0; r < 10; r++) go();
+        CUDA_TRY(cudaEventRecord(b));
+        CUDA_TRY(cudaEventSynchronize(b));
+        float ms;
+        CUDA_TRY(cudaEventElapsedTime(&ms, a, b));
+        c.ms = ms / 10;
+        if (verbose)
+          std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread (unrolled by %d): %.4f ms\n",
+                       pass == 0 ? "H" : "E", kz, unroll, c.ms);
+        if (c.ms < best_ms) {
+          best_ms = c.ms;
+          best = c;
+        }
+      }
+    }
+  }
+  cudaEventDestroy(a);
+  cudaEventDestroy(b);
+  CUDA_TRY(cudaGetLastError());
+  return FDTD_OK;
+}
+
 template <typename T>
 static fdtd_status tune_passes(fdtd_sim* s, bool time_variants) {
+  CUDA_TRY(cudaFuncSetAttribute(dft_contract<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_smem_bytes<T>()));
+  // The direct passes run unless a knob of the staged ones is set, or the
+  // grid is beyond their 32-bit cell offsets.
+  {
+    const char* force = std::getenv("FDTD_PASS");
+    const bool knobs = (force && std::strncmp(force, "flat:", 5)) || std::getenv("FDTD_TMA") || std::getenv("FDTD_PDL");
+    if (!knobs && s->ncell < ((size_t)1 << 31)) return tune_flat<T>(s, time_variants, force);
+  }
   staged_attributes<T>();
   // defaults; FDTD_PASS=staged:TY:MINB:KCHUNK[:STAGES] forces a variant,
   // FDTD_TUNE=0 skips the timing, small grids are not worth timing
@@ -1245,24 +1395,6 @@ static fdtd_status tune_passes(fdtd_sim* s, bool time_variants) {
   CUDA_TRY(cudaGetLastError());
   s->tuned = true;
   return FDTD_OK;
-}
-
-// A launch on `st` that, when pdl is set, carries a programmatic dependency
-// on the launch before it on the stream: it may start once every CTA of
-// that launch has started, and orders itself with griddepcontrol.wait.
-template <typename... P, typename... A>
-static void launch_ex(bool pdl, void (*kern)(P...), dim3 g, dim3 blk, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g;
-  cfg.blockDim = blk;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
 // The split per-half entry points (fdtd_update_h / _line / _e) launch the

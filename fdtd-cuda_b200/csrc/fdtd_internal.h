@@ -6,7 +6,8 @@
 //                      bits 3..7: dielectric class), read only inside the
 //                      material bounding box
 //   CPML psi slabs     z slabs [w][NY][PX], y slabs [NZ][w][PX],
-//                      x slabs [NZ][NY][w]; w = Ncpml (H) or Ncpml+1 (E)
+//                      x slabs [NZ][NY][W] (CpmlAxis::W); w = Ncpml (H) or
+//                      Ncpml+1 (E)
 //   dispersive cells   compact per-component lists + SoA state per slot
 //   DFT                sample ring [TB][rows] of T, accumulators
 //                      [F][rows] of double (re, im)
@@ -48,8 +49,15 @@ struct CpmlAxis {
   const T* ce_N_ey;  // ce_N used by Ey's near-x slab (reference passes ce_y_N)
   const T* inv_ked;  // 1/(kappa_e * d), length N
   const T* inv_khd;  // 1/(kappa_h * d), length N
+  // the recursion tables over every index of the axis, zero outside the
+  // slabs (padded to a multiple of 8, 16-byte aligned)
+  const T* be; const T* ce; const T* bh; const T* ch;
+  const T* ce_ey;    // ce with ce_N_ey in the near slab
   T inv_d;           // 1/d
   int Nc, F;         // slab width, first index of the far slab
+  // the x axis: psi rows of W values, the near slab's cells 0 .. Wn-1 and then
+  // the cells fb .. PX-1, both bounds multiples of a 16-byte vector
+  int W, Wn, fb;
 };
 
 // Incident-field geometry for the TFSF corrections (CORRECT_* main.cu:369).
@@ -82,6 +90,10 @@ struct SimView {
                         // line's E is double-buffered and passed per launch
   int* nonfinite;
   const SimView* self;  // a copy of this view in device memory (cold paths)
+  // this step's TFSF increments of the H and the E faces (flat.cuh), null when
+  // the TFSF launch applies the corrections
+  const T* incH;
+  const T* incE;
   int periodic;         // 1: x and y wrap around (every x and y index is updated)
 };
 

@@ -1,0 +1,463 @@
+// Direct E and H passes: the Yee updates with the CPML recursions and, for a
+// plane wave at normal incidence, the TFSF corrections, one launch per pass
+// over the whole grid.
+//
+// A field plane is contiguous in memory (NY rows of PX values), so a thread
+// takes one 16-byte vector of it (4 FP32 or 2 FP64 cells along x) counted
+// over the whole plane, whatever NX is, and KZ planes of it one after the
+// other.  Every neighbour is then a load at a constant offset (+-PX, +-plane)
+// or the next lane's register (+-1), and nothing is staged: the loads of a
+// plane do not depend on one another, and the +-1 rows and planes come out
+// of L1 and L2.
+//
+// Why this form: the passes are bound by the bytes of the six fields (9
+// values a cell and pass) at large grids and by latency at small ones.  The
+// ring of shared-memory stages (staged.cuh) walks 8 to 32 planes per CTA
+// with a barrier each; a small grid fills the GPU only for a short chain of
+// such steps, and the CPML tiles of a large one stall on their psi loads.
+#pragma once
+#include "kernels.cuh"
+
+namespace fdtd {
+
+template <typename T>
+struct alignas(16) Vec {
+  static constexpr int N = 16 / (int)sizeof(T);
+  T v[N];
+};
+template <typename T>
+__device__ __forceinline__ Vec<T> ldv(const T* p) {
+  return *reinterpret_cast<const Vec<T>*>(p);
+}
+// the same through the read-only path: values no thread of the launch writes
+__device__ __forceinline__ Vec<float> ldgv(const float* p) {
+  const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+  return Vec<float>{{x.x, x.y, x.z, x.w}};
+}
+__device__ __forceinline__ Vec<double> ldgv(const double* p) {
+  const double2 x = __ldg(reinterpret_cast<const double2*>(p));
+  return Vec<double>{{x.x, x.y}};
+}
+template <typename T>
+__device__ __forceinline__ void stv(T* p, const Vec<T>& x) {
+  *reinterpret_cast<Vec<T>*>(p) = x;
+}
+template <typename T>
+__device__ __forceinline__ Vec<T> zerov() {
+  Vec<T> r;
+#pragma unroll
+  for (int l = 0; l < Vec<T>::N; l++) r.v[l] = T(0);
+  return r;
+}
+
+constexpr int kFlatThreads = 256;
+
+// CPML of one vector and one axis: psi <- b psi + c diff / d per lane, and
+// the field += sg coef psi; w = lanes that are updated (the others keep psi).
+template <typename T>
+__device__ __forceinline__ T lane_of(const T& x, int) { return x; }
+template <typename T>
+__device__ __forceinline__ T lane_of(const Vec<T>& x, int l) { return x.v[l]; }
+template <typename T, typename C>
+__device__ __forceinline__ void psi_vec(T* p, const Vec<T>& old, const T* b, const T* c, bool per_lane, T inv_d,
+                                        const Vec<T>& diff, Vec<T>& v, T sg, const C& coef, unsigned w,
+                                        bool whole) {
+  constexpr int N = Vec<T>::N;
+  Vec<T> ps;
+#pragma unroll
+  for (int l = 0; l < N; l++) {
+    const T bl = per_lane ? b[l] : b[0], cl = per_lane ? c[l] : c[0];
+    const T x = rfma(bl, old.v[l], rmul(rmul(cl, diff.v[l]), inv_d));
+    const bool on = (w >> l) & 1;
+    ps.v[l] = on ? x : old.v[l];
+    if (on) v.v[l] = rfma(sg * lane_of(coef, l), x, v.v[l]);
+  }
+  if (whole) stv(p, ps);
+  else {
+#pragma unroll
+    for (int l = 0; l < N; l++)
+      if ((w >> l) & 1) p[l] = ps.v[l];
+  }
+}
+
+// Lanes of the vector at i0 whose cell index lies in [lo, hi).
+template <int N>
+__device__ __forceinline__ unsigned lanes_in(int i0, int lo, int hi) {
+  unsigned m = 0;
+#pragma unroll
+  for (int l = 0; l < N; l++) m |= (i0 + l >= lo && i0 + l < hi) ? 1u << l : 0u;
+  return m;
+}
+template <typename T>
+__device__ __forceinline__ void add_lanes(Vec<T>& v, unsigned m, T x) {
+#pragma unroll
+  for (int l = 0; l < Vec<T>::N; l++)
+    if ((m >> l) & 1) v.v[l] += x;
+}
+
+// The step's TFSF increments on the faces (CORRECT_X/Y/Z, main.cu:369-758) of
+// a plane wave along z: per face (axis, side) and tangential component (slot
+// 0 = the axis after the normal, 1 = the one after that) one value per z
+// index, the sign included; zero where the incident field has no such
+// component.  line_flat fills them from the 1D line (TfsfInc below).
+__host__ __device__ __forceinline__ int tfsf_inc_at(int axis, int side, int slot, int NZ) {
+  return ((axis * 2 + side) * 2 + slot) * NZ;
+}
+template <typename T>
+__device__ __forceinline__ void h_flat_tfsf(const SimView<T>& s, int i0, int j, int k, Vec<T>& hx, Vec<T>& hy,
+                                            Vec<T>& hz) {
+  constexpr int N = Vec<T>::N;
+  const int NX = s.NX, NY = s.NY, NZ = s.NZ, Tx = s.tf.Tx, Ty = s.tf.Ty, Tz = s.tf.Tz;
+  const T* inc = s.incH + k;
+  const bool kin = k >= Tz && k < NZ - Tz, kon = k >= Tz;       // half-open, closed (k <= NZ - Tz holds)
+  const bool jin = j >= Ty && j < NY - Ty, jon = j >= Ty && j <= NY - Ty;
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const int fx = side ? NX - Tx : Tx - 1, fy = side ? NY - Ty : Ty - 1, fz = side ? NZ - Tz : Tz - 1;
+    if (fx >= i0 && fx < i0 + N) {
+      const unsigned m = 1u << (fx - i0);
+      if (jon && kin) add_lanes(hy, m, inc[tfsf_inc_at(0, side, 0, NZ)]);
+      if (jin && kon) add_lanes(hz, m, inc[tfsf_inc_at(0, side, 1, NZ)]);
+    }
+    if (j == fy) {
+      if (kon) add_lanes(hz, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(1, side, 0, NZ)]);
+      if (kin) add_lanes(hx, lanes_in<N>(i0, Tx, NX - Tx + 1), inc[tfsf_inc_at(1, side, 1, NZ)]);
+    }
+    if (k == fz) {
+      if (jin) add_lanes(hx, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), inc[tfsf_inc_at(2, side, 0, NZ)]);
+      if (jon) add_lanes(hy, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(2, side, 1, NZ)]);
+    }
+  }
+}
+// The E half, added to E before its update; axis by axis (an edge cell takes
+// two corrections, in the order X, Y, Z).
+template <typename T>
+__device__ __forceinline__ void e_flat_tfsf(const SimView<T>& s, int i0, int j, int k, Vec<T>& ex, Vec<T>& ey,
+                                            Vec<T>& ez) {
+  constexpr int N = Vec<T>::N;
+  const int NX = s.NX, NY = s.NY, NZ = s.NZ, Tx = s.tf.Tx, Ty = s.tf.Ty, Tz = s.tf.Tz;
+  const T* inc = s.incE + k;
+  const bool kin = k < NZ - Tz;  // Tz <= k <= NZ - Tz holds
+  const bool jin = j >= Ty && j < NY - Ty, jon = j >= Ty && j <= NY - Ty;
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const int fx = side ? NX - Tx : Tx;
+    if (fx >= i0 && fx < i0 + N) {
+      const unsigned m = 1u << (fx - i0);
+      if (jin) add_lanes(ey, m, inc[tfsf_inc_at(0, side, 0, NZ)]);
+      if (jon && kin) add_lanes(ez, m, inc[tfsf_inc_at(0, side, 1, NZ)]);
+    }
+  }
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const int fy = side ? NY - Ty : Ty;
+    if (j == fy) {
+      if (kin) add_lanes(ez, lanes_in<N>(i0, Tx, NX - Tx + 1), inc[tfsf_inc_at(1, side, 0, NZ)]);
+      add_lanes(ex, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(1, side, 1, NZ)]);
+    }
+  }
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const int fz = side ? NZ - Tz : Tz;
+    if (k == fz) {
+      if (jon) add_lanes(ex, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(2, side, 0, NZ)]);
+      if (jin) add_lanes(ey, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), inc[tfsf_inc_at(2, side, 1, NZ)]);
+    }
+  }
+}
+
+// H pass (UPDATE_hx/hy/hz, main.cu:762-1044) of the vector vq of the plane,
+// planes k0 .. k0+KZ-1.  Same arithmetic and order per cell as h_pass_tile
+// (staged.cuh); the H half of CORRECT_X/Y/Z is added to the updated value
+// from the step's increments (incH) when the view carries them.
+template <typename T, int U>
+__device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, int k0, int kz) {
+  constexpr int N = Vec<T>::N;
+  const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
+  const unsigned PXV = (unsigned)PX / N, NV = PXV * (unsigned)NY;
+  const bool in = vq < NV;
+  if (!in) vq = NV - 1;  // takes part in the shuffles, stores nothing
+  const int j = (int)(vq / PXV), i0 = (int)(vq - (unsigned)j * PXV) * N;
+  const unsigned plane = (unsigned)s.plane, c0 = vq * N;  // 32-bit cell offsets (the host checks the range)
+  const bool per = s.periodic != 0;
+  const bool hasy = per || j + 1 < NY;
+  // offset of the +y row; the last row of a bounded grid reads itself (its
+  // hx and hz are not updated)
+  const int oj = j + 1 < NY ? PX : (per ? -(NY - 1) * PX : 0);
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned wx = lanes_in<N>(i0, 0, per ? NX : NX - 1);  // lanes with a +x neighbour
+  const Vec<T> ikx = ldgv(s.cp[0].inv_khd + i0);
+  const T iky = ldg(s.cp[1].inv_khd + j);
+  const T che = s.che, chh = s.chh;
+  // CPML slabs of this vector
+  const int xs = s.cp[0].Nc <= 0 ? -1 : i0 < s.cp[0].Wn ? i0 : (i0 + N > s.cp[0].fb ? i0 - s.cp[0].fb + s.cp[0].Wn : -1);
+  const bool yfar = j >= s.cp[1].F;
+  const int ys = s.cp[1].Nc <= 0 ? -1 : j < s.cp[1].Nc ? j : (yfar && j < NY - 1 ? j - s.cp[1].F : -1);
+  const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
+  // next vector's first value along x, from the next lane
+  const bool edge = lane == 31 || i0 + N >= PX;
+  const int ox = i0 + N < PX ? N : (per ? N - PX : 0);
+  const TfsfView& tf = s.tf;
+  const bool tfsf = s.incH != nullptr;
+  const unsigned b0 = (unsigned)k0 * plane + c0;
+  Vec<T> ex = ldgv(s.E[0] + b0), ey = ldgv(s.E[1] + b0);
+  const int k1 = min(k0 + kz, NZ);
+#pragma unroll U
+  for (int k = k0; k < k1; k++) {
+    const unsigned b = (unsigned)k * plane + c0;
+    const bool hask = k + 1 < NZ;
+    const unsigned bn = hask ? b + plane : b;
+    // every load of the plane
+    const Vec<T> ez = ldgv(s.E[2] + b);
+    const Vec<T> exn = ldgv(s.E[0] + bn), eyn = ldgv(s.E[1] + bn);
+    const Vec<T> exj = ldgv(s.E[0] + b + oj), ezj = ldgv(s.E[2] + b + oj);
+    Vec<T> hx = ldv(s.H[0] + b), hy = ldv(s.H[1] + b), hz = ldv(s.H[2] + b);
+    T eyi = T(0), ezi = T(0);
+    if (edge) { eyi = ldg(s.E[1] + b + ox); ezi = ldg(s.E[2] + b + ox); }
+    const T ikz = ldg(s.cp[2].inv_khd + k);
+    T *px0 = nullptr, *px1 = nullptr, *py0 = nullptr, *py1 = nullptr, *pz0 = nullptr, *pz1 = nullptr;
+    Vec<T> ox0, ox1, oy0, oy1, oz0, oz1;
+    int zs = -1;
+    if (hask && Ncz > 0) zs = k < Ncz ? k : (k >= Fz ? k - Fz + Ncz : -1);
+    if (zs >= 0) {
+      const unsigned o = (unsigned)zs * plane + c0;
+      pz0 = s.psiH_N[0][1] + o; pz1 = s.psiH_N[1][0] + o;
+      oz0 = ldv(pz0); oz1 = ldv(pz1);
+    }
+    if (xs >= 0 && hask) {
+      const unsigned o = ((unsigned)k * NY + j) * s.cp[0].W + xs;
+      px0 = s.psiH_N[1][1] + o; px1 = s.psiH_N[2][0] + o;
+      ox0 = ldv(px0); ox1 = ldv(px1);
+    }
+    if (ys >= 0 && hask) {
+      const unsigned o = ((unsigned)k * s.cp[1].Nc + ys) * PX + i0;
+      py0 = (yfar ? s.psiH_F[0][0] : s.psiH_N[0][0]) + o;
+      py1 = (yfar ? s.psiH_F[2][1] : s.psiH_N[2][1]) + o;
+      oy0 = ldv(py0); oy1 = ldv(py1);
+    }
+    {
+      const T a = __shfl_down_sync(0xFFFFFFFFu, ey.v[0], 1), c = __shfl_down_sync(0xFFFFFFFFu, ez.v[0], 1);
+      if (!edge) { eyi = a; ezi = c; }
+    }
+    // differences
+    Vec<T> dzy, dzx, dyz, dyx, dxz, dxy;  // d(ey)/dz, d(ex)/dz, d(ez)/dy, d(ex)/dy, d(ez)/dx, d(ey)/dx
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      dzy.v[l] = rsub(eyn.v[l], ey.v[l]);
+      dzx.v[l] = rsub(exn.v[l], ex.v[l]);
+      dyz.v[l] = rsub(ezj.v[l], ez.v[l]);
+      dyx.v[l] = rsub(exj.v[l], ex.v[l]);
+      dxz.v[l] = rsub(l + 1 < N ? ez.v[l + 1 < N ? l + 1 : 0] : ezi, ez.v[l]);
+      dxy.v[l] = rsub(l + 1 < N ? ey.v[l + 1 < N ? l + 1 : 0] : eyi, ey.v[l]);
+    }
+    Vec<T> vx, vy, vz;
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      vx.v[l] = rfma(che, rcurl(dzy.v[l], ikz, dyz.v[l], iky), rmul(chh, hx.v[l]));
+      vy.v[l] = rfma(che, rcurl(dxz.v[l], ikx.v[l], dzx.v[l], ikz), rmul(chh, hy.v[l]));
+      vz.v[l] = rfma(che, rcurl(dyx.v[l], iky, dxy.v[l], ikx.v[l]), rmul(chh, hz.v[l]));
+    }
+    // CPML (cells with every index below N-1, main.cu:829); per axis in the
+    // order z, x, y
+    const unsigned wp = hasy && in ? wx : 0u;
+    if (wp) {
+      if (zs >= 0) {
+        const T bz = ldg(s.cp[2].bh + k), cz = ldg(s.cp[2].ch + k);
+        psi_vec(pz0, oz0, &bz, &cz, false, s.cp[2].inv_d, dzy, vx, T(1), che, wp, true);
+        psi_vec(pz1, oz1, &bz, &cz, false, s.cp[2].inv_d, dzx, vy, T(-1), che, wp, true);
+      }
+      if (xs >= 0 && hask) {
+        const Vec<T> bx = ldgv(s.cp[0].bh + i0), cx = ldgv(s.cp[0].ch + i0);
+        psi_vec(px0, ox0, bx.v, cx.v, true, s.cp[0].inv_d, dxz, vy, T(1), che, wp, true);
+        psi_vec(px1, ox1, bx.v, cx.v, true, s.cp[0].inv_d, dxy, vz, T(-1), che, wp, true);
+      }
+      if (ys >= 0 && hask) {
+        const T by = ldg(s.cp[1].bh + j), cy = ldg(s.cp[1].ch + j);
+        psi_vec(py0, oy0, &by, &cy, false, s.cp[1].inv_d, dyz, vx, T(-1), che, wp, true);
+        psi_vec(py1, oy1, &by, &cy, false, s.cp[1].inv_d, dyx, vz, T(1), che, wp, true);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      const bool on = (wx >> l) & 1;
+      hx.v[l] = vx.v[l];
+      if (on) { hy.v[l] = vy.v[l]; hz.v[l] = vz.v[l]; }
+    }
+    if (tfsf && k >= tf.Tz - 1 && k <= NZ - tf.Tz) h_flat_tfsf(s, i0, j, k, hx, hy, hz);
+    if (in) {
+      if (hasy && hask) stv(s.H[0] + b, hx);
+      if (hask) stv(s.H[1] + b, hy);
+      if (hasy) stv(s.H[2] + b, hz);
+    }
+    ex = exn;
+    ey = eyn;
+  }
+}
+
+template <typename T, int U>
+__global__ void __launch_bounds__(kFlatThreads, 2) h_flat(const __grid_constant__ SimView<T> s, unsigned nbx, int kz) {
+  pdl_launch_dependents();
+  const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
+  h_flat_cells<T, U>(s, xb * kFlatThreads + threadIdx.x, (int)kb * kz, kz);
+  pdl_wait();
+}
+
+// E pass (UPDATE_ex/ey/ez, main.cu:1048-1912) of the vector vq, planes k0 ..
+// k0+KZ-1: e_pass_tile's arithmetic and order per cell (CPML per axis in the
+// order z, y, x).  The E half of CORRECT_X/Y/Z goes in before the update.
+// Dispersive components are left to the dispersive-cell kernels, which run
+// beside this one: a vector with such a cell stores lane by lane.
+template <typename T, int U>
+__device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, int k0, int kz) {
+  constexpr int N = Vec<T>::N;
+  const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
+  const unsigned PXV = (unsigned)PX / N, NV = PXV * (unsigned)NY;
+  const bool in = vq < NV;
+  if (!in) vq = NV - 1;
+  const int j = (int)(vq / PXV), i0 = (int)(vq - (unsigned)j * PXV) * N;
+  const unsigned plane = (unsigned)s.plane, c0 = vq * N;
+  const bool per = s.periodic != 0;
+  const int oj = j > 0 ? -PX : (per ? (NY - 1) * PX : 0);
+  const unsigned lane = threadIdx.x & 31;
+  // lanes whose ex, ey, ez are updated in this column (main.cu:1172, 1476,
+  // 1767; every column when periodic, main.cu:1072, 1364, 1668)
+  const bool jlo = per || j > 0, jhi = per || j < NY - 1;
+  const unsigned wlo = per ? lanes_in<N>(i0, 0, NX) : lanes_in<N>(i0, 1, NX - 1);
+  const unsigned wall = per ? wlo : lanes_in<N>(i0, 0, NX - 1);
+  const unsigned cx = in && jlo && jhi ? wall : 0u, cy = in && jhi ? wlo : 0u, cz = in && jlo && jhi ? wlo : 0u;
+  const Vec<T> ikx = ldgv(s.cp[0].inv_ked + i0);
+  const T iky = ldg(s.cp[1].inv_ked + j);
+  const T cee0 = s.cee[0], ceh0 = s.ceh[0];
+  const bool inbox = i0 + N > s.mat_lo[0] && i0 < s.mat_hi[0] && j >= s.mat_lo[1] && j < s.mat_hi[1];
+  const int xs = s.cp[0].Nc <= 0 ? -1 : i0 < s.cp[0].Wn ? i0 : (i0 + N > s.cp[0].fb ? i0 - s.cp[0].fb + s.cp[0].Wn : -1);
+  const bool yfar = j >= s.cp[1].F;
+  const int ys = s.cp[1].Nc <= 0 ? -1 : j <= s.cp[1].Nc ? j : (yfar ? j - s.cp[1].F : -1);
+  const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
+  const bool edge = lane == 0 || i0 == 0;
+  const int ox = i0 > 0 ? -1 : (per ? PX - 1 : 0);
+  const bool tfsf = s.incE != nullptr;
+  T check = T(0);
+  const unsigned bm = (unsigned)max(k0 - 1, 0) * plane + c0;
+  Vec<T> hxm = ldgv(s.H[0] + bm), hym = ldgv(s.H[1] + bm);
+  const int k1 = min(k0 + kz, NZ);
+#pragma unroll U
+  for (int k = k0; k < k1; k++) {
+    const unsigned b = (unsigned)k * plane + c0;
+    const bool okz = k < NZ - 1, hasz = k > 0;
+    // every load of the plane
+    const Vec<T> hx = ldgv(s.H[0] + b), hy = ldgv(s.H[1] + b), hz = ldgv(s.H[2] + b);
+    const Vec<T> hxj = ldgv(s.H[0] + b + oj), hzj = ldgv(s.H[2] + b + oj);
+    Vec<T> ex = ldv(s.E[0] + b), ey = ldv(s.E[1] + b), ez = ldv(s.E[2] + b);
+    T hyi = T(0), hzi = T(0);
+    if (edge) { hyi = ldg(s.H[1] + b + ox); hzi = ldg(s.H[2] + b + ox); }
+    const T ikz = ldg(s.cp[2].inv_ked + k);
+    T *px0 = nullptr, *px1 = nullptr, *py0 = nullptr, *py1 = nullptr, *pz0 = nullptr, *pz1 = nullptr;
+    Vec<T> ox0, ox1, oy0, oy1, oz0, oz1;
+    int zs = -1;
+    if (okz && Ncz > 0) zs = k <= Ncz ? k : (k >= Fz ? k - Fz + Ncz + 1 : -1);
+    if (zs >= 0) {
+      const unsigned o = (unsigned)zs * plane + c0;
+      pz0 = s.psiE_N[0][1] + o; pz1 = s.psiE_N[1][0] + o;
+      oz0 = ldv(pz0); oz1 = ldv(pz1);
+    }
+    if (ys >= 0 && okz) {
+      const unsigned o = ((unsigned)k * (s.cp[1].Nc + 1) + ys) * PX + i0;
+      py0 = (yfar ? s.psiE_F[0][0] : s.psiE_N[0][0]) + o;
+      py1 = (yfar ? s.psiE_F[2][1] : s.psiE_N[2][1]) + o;
+      oy0 = ldv(py0); oy1 = ldv(py1);
+    }
+    if (xs >= 0 && okz) {
+      const unsigned o = ((unsigned)k * NY + j) * s.cp[0].W + xs;
+      px0 = s.psiE_N[1][1] + o; px1 = s.psiE_N[2][0] + o;
+      ox0 = ldv(px0); ox1 = ldv(px1);
+    }
+    // dielectric classes and dispersive components
+    Vec<T> ceh;
+    unsigned mx = 0, my = 0, mz = 0;
+#pragma unroll
+    for (int l = 0; l < N; l++) ceh.v[l] = ceh0;
+    if (inbox && k >= s.mat_lo[2] && k < s.mat_hi[2]) {
+      const uint8_t* mp = s.mat + b;
+#pragma unroll
+      for (int l = 0; l < N; l++) {
+        const unsigned m = mp[l];
+        mx |= (m & 1u) << l;
+        my |= ((m >> 1) & 1u) << l;
+        mz |= ((m >> 2) & 1u) << l;
+        if (m >> 3) ceh.v[l] = s.ceh[m >> 3];
+      }
+    }
+    {
+      const T a = __shfl_up_sync(0xFFFFFFFFu, hy.v[N - 1], 1), c = __shfl_up_sync(0xFFFFFFFFu, hz.v[N - 1], 1);
+      if (!edge) { hyi = a; hzi = c; }
+    }
+    const unsigned wx = hasz && okz ? cx & ~mx : 0u, wy = hasz && okz ? cy & ~my : 0u, wz = okz ? cz & ~mz : 0u;
+    const bool whole = (mx | my | mz) == 0;
+    if (tfsf && k >= s.tf.Tz && k <= NZ - s.tf.Tz) e_flat_tfsf(s, i0, j, k, ex, ey, ez);
+    Vec<T> dyz, dzy, dzx, dxz, dxy, dyx;  // d(hz)/dy, d(hy)/dz, d(hx)/dz, d(hz)/dx, d(hy)/dx, d(hx)/dy
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      dyz.v[l] = rsub(hz.v[l], hzj.v[l]);
+      dzy.v[l] = rsub(hy.v[l], hym.v[l]);
+      dzx.v[l] = rsub(hx.v[l], hxm.v[l]);
+      dxz.v[l] = rsub(hz.v[l], l > 0 ? hz.v[l > 0 ? l - 1 : 0] : hzi);
+      dxy.v[l] = rsub(hy.v[l], l > 0 ? hy.v[l > 0 ? l - 1 : 0] : hyi);
+      dyx.v[l] = rsub(hx.v[l], hxj.v[l]);
+    }
+    Vec<T> vx, vy, vz;
+#pragma unroll
+    for (int l = 0; l < N; l++) {
+      vx.v[l] = rfma(ceh.v[l], rcurl(dyz.v[l], iky, dzy.v[l], ikz), rmul(cee0, ex.v[l]));
+      vy.v[l] = rfma(ceh.v[l], rcurl(dzx.v[l], ikz, dxz.v[l], ikx.v[l]), rmul(cee0, ey.v[l]));
+      vz.v[l] = rfma(ceh.v[l], rcurl(dxy.v[l], ikx.v[l], dyx.v[l], iky), rmul(cee0, ez.v[l]));
+    }
+    // CPML (cells with i < NX-1, j < NY-1, k < NZ-1: the masks hold these)
+    if (zs >= 0) {
+      const T bz = ldg(s.cp[2].be + k), cc = ldg(s.cp[2].ce + k);
+      if (wx) psi_vec(pz0, oz0, &bz, &cc, false, s.cp[2].inv_d, dzy, vx, T(-1), ceh, wx, whole);
+      if (wy) psi_vec(pz1, oz1, &bz, &cc, false, s.cp[2].inv_d, dzx, vy, T(1), ceh, wy, whole);
+    }
+    if (ys >= 0 && okz) {
+      const T by = ldg(s.cp[1].be + j), cc = ldg(s.cp[1].ce + j);
+      if (wx) psi_vec(py0, oy0, &by, &cc, false, s.cp[1].inv_d, dyz, vx, T(1), ceh, wx, whole);
+      if (wz) psi_vec(py1, oy1, &by, &cc, false, s.cp[1].inv_d, dyx, vz, T(-1), ceh, wz, whole);
+    }
+    if (xs >= 0 && okz) {
+      const Vec<T> bx = ldgv(s.cp[0].be + i0), cc = ldgv(s.cp[0].ce + i0), cy_ = ldgv(s.cp[0].ce_ey + i0);
+      if (wy) psi_vec(px0, ox0, bx.v, cy_.v, true, s.cp[0].inv_d, dxz, vy, T(-1), ceh, wy, whole);
+      if (wz) psi_vec(px1, ox1, bx.v, cc.v, true, s.cp[0].inv_d, dxy, vz, T(1), ceh, wz, whole);
+    }
+    if (whole) {
+#pragma unroll
+      for (int l = 0; l < N; l++) {
+        if ((wx >> l) & 1) { ex.v[l] = vx.v[l]; check += vx.v[l]; }
+        if ((wy >> l) & 1) { ey.v[l] = vy.v[l]; check += vy.v[l]; }
+        if ((wz >> l) & 1) { ez.v[l] = vz.v[l]; check += vz.v[l]; }
+      }
+      if (wx) stv(s.E[0] + b, ex);
+      if (wy) stv(s.E[1] + b, ey);
+      if (wz) stv(s.E[2] + b, ez);
+    } else {
+#pragma unroll
+      for (int l = 0; l < N; l++) {
+        if ((wx >> l) & 1) { s.E[0][b + l] = vx.v[l]; check += vx.v[l]; }
+        if ((wy >> l) & 1) { s.E[1][b + l] = vy.v[l]; check += vy.v[l]; }
+        if ((wz >> l) & 1) { s.E[2][b + l] = vz.v[l]; check += vz.v[l]; }
+      }
+    }
+    hxm = hx;
+    hym = hy;
+  }
+  // NaN/Inf watchdog: a non-finite value makes the running sum non-finite
+  if (!isfinite(check)) atomicOr(s.nonfinite, 1);
+}
+
+template <typename T, int U>
+__global__ void __launch_bounds__(kFlatThreads, 2) e_flat(const __grid_constant__ SimView<T> s, unsigned nbx, int kz) {
+  pdl_launch_dependents();
+  const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
+  e_flat_cells<T, U>(s, xb * kFlatThreads + threadIdx.x, (int)kb * kz, kz);
+  pdl_wait();
+}
+
+}  // namespace fdtd

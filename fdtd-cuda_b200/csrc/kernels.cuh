@@ -202,7 +202,8 @@ __device__ __forceinline__ void tfsf_e_walk(const SimView<T>& s, int c, int i, i
 
 // ---------------------------------------------------------------------
 // CPML psi helpers.  psi layouts: z slab [w][NY][PX], y slab [NZ][w][PX],
-// x slab [NZ][NY][w].
+// x slab [NZ][NY][W] with the near cells first (CpmlAxis).  slab_idx with
+// ax = 0 is the adjoint's own x layout [NZ][NY][w].
 
 template <typename T>
 __device__ __forceinline__ size_t slab_idx(const SimView<T>& s, int ax, int w, int i, int j, int k) {
@@ -222,15 +223,15 @@ __device__ __forceinline__ T cpml_e(const SimView<T>& s, int c, int slot, int ax
   int near_lim = (c == 2 && ax == 1) ? a.Nc : a.Nc + 1;
   if (q < near_lim) {
     const T* ceN = (c == 1 && ax == 0) ? a.ce_N_ey : a.ce_N;
-    T* p = s.psiE_N[c][slot] + slab_idx(s, ax, a.Nc + 1, i, j, k);
+    T* p = s.psiE_N[c][slot] + slab_idx(s, ax, ax == 0 ? a.W : a.Nc + 1, i, j, k);
     T ps = ldg(a.be_N + q) * *p + ldg(ceN + q) * diff * a.inv_d;
     *p = ps;
     v += sg * (ceh * ps);
   }
   if (q >= a.F) {
     int q2 = q - a.F;
-    int ii = ax == 0 ? q2 : i, jj = ax == 1 ? q2 : j, kk = ax == 2 ? q2 : k;
-    T* p = s.psiE_F[c][slot] + slab_idx(s, ax, a.Nc + 1, ii, jj, kk);
+    int ii = ax == 0 ? i - a.fb : i, jj = ax == 1 ? q2 : j, kk = ax == 2 ? q2 : k;
+    T* p = s.psiE_F[c][slot] + slab_idx(s, ax, ax == 0 ? a.W : a.Nc + 1, ii, jj, kk);
     T ps = ldg(a.be_F + q2) * *p + ldg(a.ce_F + q2) * diff * a.inv_d;
     *p = ps;
     v += sg * (ceh * ps);

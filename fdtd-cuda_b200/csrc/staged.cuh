@@ -394,14 +394,14 @@ __device__ __forceinline__ void h_pass_tile(const SimView<T>& s, int kchunk, int
   const T idx_ = s.cp[0].inv_d, idy_ = s.cp[1].inv_d, idz_ = s.cp[2].inv_d;
   const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
   // psi offsets in 32 bits; near and far slabs are contiguous (near first)
-  const unsigned xstep = (unsigned)NY * (unsigned)s.cp[0].Nc, ystep = (unsigned)s.cp[1].Nc * (unsigned)PX;
+  const unsigned xstep = (unsigned)NY * (unsigned)s.cp[0].W, ystep = (unsigned)s.cp[1].Nc * (unsigned)PX;
   const unsigned plane32 = (unsigned)plane, jrow = (unsigned)j * (unsigned)PX + (unsigned)i;
   T* bx0 = nullptr;  // psi_hy(x) at plane 0
   T* bx1 = nullptr;  // psi_hz(x)
   T* by0 = nullptr;  // psi_hx(y)
   T* by1 = nullptr;  // psi_hz(y)
   if (sx.side) {
-    const size_t q = (size_t)j * s.cp[0].Nc + sx.q;
+    const size_t q = (size_t)j * s.cp[0].W + (sx.side == 1 ? i : i - s.cp[0].fb);
     bx0 = (sx.side == 1 ? s.psiH_N[1][1] : s.psiH_F[1][1]) + q;
     bx1 = (sx.side == 1 ? s.psiH_N[2][0] : s.psiH_F[2][0]) + q;
   }
@@ -634,14 +634,14 @@ __device__ __forceinline__ void e_pass_tile(const SimView<T>& s, int kchunk, int
   const T idx_ = s.cp[0].inv_d, idy_ = s.cp[1].inv_d, idz_ = s.cp[2].inv_d;
   const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
   // psi offsets in 32 bits; near and far slabs are contiguous (near first)
-  const unsigned xstep = (unsigned)NY * (unsigned)(s.cp[0].Nc + 1), ystep = (unsigned)(s.cp[1].Nc + 1) * (unsigned)PX;
+  const unsigned xstep = (unsigned)NY * (unsigned)s.cp[0].W, ystep = (unsigned)(s.cp[1].Nc + 1) * (unsigned)PX;
   const unsigned plane32 = (unsigned)plane, jrow = (unsigned)j * (unsigned)PX + (unsigned)i;
   T* bx0 = nullptr;  // psi_ey(x) at plane 0
   T* bx1 = nullptr;  // psi_ez(x)
   T* by0 = nullptr;  // psi_ex(y)
   T* by1 = nullptr;  // psi_ez(y)
   if (sx.side) {
-    const size_t q = (size_t)j * (s.cp[0].Nc + 1) + sx.q;
+    const size_t q = (size_t)j * s.cp[0].W + (sx.side == 1 ? i : i - s.cp[0].fb);
     bx0 = (sx.side == 1 ? s.psiE_N[1][1] : s.psiE_F[1][1]) + q;
     bx1 = (sx.side == 1 ? s.psiE_N[2][0] : s.psiE_F[2][0]) + q;
   }

@@ -1,0 +1,73 @@
+"""The direct E and H passes (flat.cuh) against the staged ones.
+
+Both forms do the same operations in the same order per cell, so fields are
+bit-identical: over row lengths of every remainder of the 16-byte vector and
+of the padded pitch, grids of fewer planes than a thread takes, dispersive
+cells inside the CPML, dielectric classes and periodic x and y.
+"""
+import numpy as np
+import pytest
+
+import fdtd_b200 as F
+from cases import make
+
+pytestmark = pytest.mark.gpu
+
+SPECS = ("flat:1", "flat:5", "flat:8:8", "flat:64:8", "flat:200")
+
+
+def fields(name, prec, spec, monkeypatch, steps, **over):
+    monkeypatch.setenv("FDTD_PASS", spec)
+    s = F.Sim(make(F, name, precision=prec, **over))
+    assert s.stats().h_staged == s.stats().e_staged == int(spec.startswith("staged"))
+    s.step(steps)
+    s.check()
+    out = [s.field(c) for c in range(6)]
+    spectra = s.reflectance() if s.params.periodic_xy else s.spectra()
+    s.close()
+    return out, spectra
+
+
+def agree(name, prec, specs, monkeypatch, steps=150, **over):
+    ref, tab = fields(name, prec, "staged:4:1:16:4", monkeypatch, steps, **over)
+    assert max(np.abs(f).max() for f in ref) > 0
+    for spec in specs:
+        got, t = fields(name, prec, spec, monkeypatch, steps, **over)
+        for c in range(6):
+            np.testing.assert_array_equal(got[c], ref[c], err_msg=f"{name} {spec} component {c}")
+        np.testing.assert_array_equal(t, tab)
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+@pytest.mark.parametrize("name", ["sphere_big", "slab", "disks_slab", "hydro", "fixes", "periodic_spheres"])
+def test_direct_passes_agree_with_the_staged_ones(name, prec, monkeypatch):
+    agree(name, prec, SPECS, monkeypatch)
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+@pytest.mark.parametrize("dx", range(8))
+def test_every_row_remainder(dx, prec, monkeypatch):
+    agree("sphere_au", prec, ("flat:1", "flat:7:8"), monkeypatch, steps=90, NCELLX=21 + dx, NCELLY=22 - dx % 3)
+
+
+def test_tuned_and_untuned_direct_passes_agree(monkeypatch):
+    """The shape the tuner keeps and the untimed rule's."""
+    out = []
+    for tune in ("1", "0"):
+        monkeypatch.setenv("FDTD_TUNE", tune)
+        s = F.Sim(make(F, "sphere_big", precision=F.FDTD_FP32))
+        st = s.stats()
+        assert st.h_staged == 0 and st.h_kchunk >= 1 and (st.h_ms > 0) == (tune == "1")
+        s.step(140)
+        out.append([s.field(c) for c in range(6)])
+        s.close()
+    for c in range(6):
+        np.testing.assert_array_equal(out[0][c], out[1][c])
+
+
+def test_unbuilt_direct_variant_is_rejected(monkeypatch):
+    for spec in ("flat:0", "flat:4:3"):
+        monkeypatch.setenv("FDTD_PASS", spec)
+        with pytest.raises(F.FdtdError) as e:
+            F.Sim(make(F, "vacuum", precision=F.FDTD_FP32))
+        assert e.value.status == 1 and "not built" in str(e.value)
