@@ -48,12 +48,15 @@ __global__ void tfsf_apply_batch(const BatchSim<T>* __restrict__ b) {
 template <typename T>
 __global__ void __launch_bounds__(1024) line_step_batch(const BatchSim<T>* __restrict__ b) {
   const BatchSim<T>& x = b[blockIdx.y];
-  line_step_body(x.line, x.v, x.probe_id);
+  const int t = x.clk->t;
+  __syncthreads();
+  line_step_body(x.line, x.v, x.probe_id, t);
+  if (threadIdx.x == 0) x.clk->th = t + 1;
 }
 template <typename T>
 __global__ void metal_e_batch(const BatchSim<T>* __restrict__ b) {
   const BatchSim<T>& x = b[blockIdx.y];
-  metal_e_body(x.v, x.m, x.clk);
+  metal_e_cell(x.v, x.m, x.clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
 }
 template <typename T>
 __global__ void dft_sample_batch(const BatchSim<T>* __restrict__ b) {

@@ -1,4 +1,6 @@
-// TFSF work of the time step, on the cells that need it only:
+// TFSF work of the time step as launches of its own, on the cells that need it
+// only (oblique incidence and the staged passes; at normal incidence the direct
+// passes add the corrections themselves):
 //   tfsf_tabulate                 at create: the corrections of CORRECT_X/Y/Z
 //                                 (main.cu:369-758) on the TFSF box faces
 //   tfsf_h_apply / tfsf_e_apply   every step: after the H update for H,

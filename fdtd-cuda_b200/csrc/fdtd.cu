@@ -79,8 +79,9 @@ struct fdtd_sim {
   // pdl = 1: the edge and interior launches of a pass go on one stream
   // with a programmatic dependency instead of on two streams
   struct PassCfg { int minb = 1, ty = 4, kchunk = 16, staged = 1, stages = 4, eminb = 1, estages = 4, pdl = 0, tma = 0, etma = 0; float ms = 0;
-    // direct pass (flat.cuh): planes per thread and unrolled planes; kz = 0 = the staged pass
-    int kz = 0, unroll = 1; };
+    // direct pass (flat.cuh): planes per thread, and whether they are copied
+    // ahead into shared memory; kz = 0 = the staged pass
+    int kz = 0, ring = 0; };
   // pass tiles for one (tile height, z-chunk): the interior box of tiles
   // that touch no CPML slab and the table of the others
   struct TileSet {
@@ -100,6 +101,10 @@ struct fdtd_sim {
   int tma_avail = -1;  // -1 not yet known
   ShellCells shell_h, shell_e;
   TfsfTable tf_h{}, tf_e{};  // tabulated TFSF corrections of the two shells
+  // the corrections as increments of the passes (normal incidence): the terms
+  // the line step evaluates, and whether every correction is covered
+  std::vector<TfsfInc> incs;
+  bool inc_ok = true, fused_tfsf = false;
   const void* dview = nullptr;  // device copy of the view
   PassCfg hcfg, ecfg;
   bool tuned = false;
@@ -435,24 +440,26 @@ static fdtd_status build_views(fdtd_sim* s) {
   v.periodic = su.p.periodic_xy ? 1 : 0;
   v.h_inc = s->h_inc;
   v.nonfinite = &s->clk->nonfinite;
+  v.clk = s->clk;
+  v.incH = v.incE = nullptr;  // create_impl sets them where the passes apply the TFSF
   // dispersive cells
   for (int c = 0; c < 3; c++) { m.n[c] = s->nmetal[c]; m.cell[c] = s->mcell[c]; }
   size_t maxn = std::max(s->nmetal[0], std::max(s->nmetal[1], s->nmetal[2]));
   if (maxn > 0) {
-    // per component: en, en1 in T; cpn[2], cpn1[2], pd[3], nd[2] in FP64
+    // per component: en, en1 in T; cpn[2], cpn1[2], pd[3], nd[3] in FP64
     T* st;
     double* sd;
     cudaError_t e = s->alloc(&st, (size_t)3 * 2 * maxn, true);
-    if (e == cudaSuccess) e = s->alloc(&sd, (size_t)3 * 9 * maxn, true);
+    if (e == cudaSuccess) e = s->alloc(&sd, (size_t)3 * 10 * maxn, true);
     if (e != cudaSuccess) return fail(FDTD_ERR_ALLOC, cudaGetErrorString(e));
     for (int c = 0; c < 3; c++) {
       T* b = st + (size_t)c * 2 * maxn;
-      double* d = sd + (size_t)c * 9 * maxn;
+      double* d = sd + (size_t)c * 10 * maxn;
       m.en[c] = b; m.en1[c] = b + maxn;
       m.cpn[c][0] = d; m.cpn[c][1] = d + maxn;
       m.cpn1[c][0] = d + 2 * maxn; m.cpn1[c][1] = d + 3 * maxn;
       m.pd[c][0] = d + 4 * maxn; m.pd[c][1] = d + 5 * maxn; m.pd[c][2] = d + 6 * maxn;
-      m.nd[c][0] = d + 7 * maxn; m.nd[c][1] = d + 8 * maxn;
+      m.nd[c][0] = d + 7 * maxn; m.nd[c][1] = d + 8 * maxn; m.nd[c][2] = d + 9 * maxn;
       m.nbr[c] = s->nbr[c];
     }
   }
@@ -550,12 +557,32 @@ static fdtd_status build_tfsf_table(fdtd_sim* s, const ShellCells& sh, int efiel
     seen.emplace(key, k);
     return k;
   };
+  std::vector<int> inc_at((size_t)12 * s->NZ, -1);
   for (size_t q = 0; q < n; q++) {
     const unsigned nt = (hcn[q] >> 2) & 3;
     if (nt == 0) continue;
     if (nt > 2) return fail(FDTD_ERR_INVALID, "a TFSF face cell has more than two corrections");
     const unsigned t0 = term_of(q, 0), t1 = nt > 1 ? term_of(q, 1) : t0;
     ent.push_back(make_uint4(hid[q], t0, t1, hcn[q]));
+    // the same terms as increments per face, component and z index
+    // (tfsf_inc_at): one term per entry when it depends on z alone
+    const int cell[3] = {(int)(hid[q] % s->PX), (int)(hid[q] / s->PX % s->NY), (int)(hid[q] / s->plane)};
+    const int N3[3] = {s->NX, s->NY, s->NZ}, c = (int)(hcn[q] & 3);
+    for (unsigned t = 0; t < nt && s->inc_ok; t++) {
+      const int ax = (hm[t][q] >> 1) & 3, lo = s->su.Nt[ax] - (efield ? 0 : 1), hi = N3[ax] - s->su.Nt[ax];
+      const int side = cell[ax] == hi ? 1 : 0, slot = (c - ax + 3) % 3 - 1;
+      if ((cell[ax] != lo && cell[ax] != hi) || slot < 0 || (ax < 2 && c != 2)) { s->inc_ok = false; break; }
+      const TfsfInc x{hdp[t][q], hix[t][q], (int)hm[t][q] | efield << 5 | (int)(hcn[q] >> 8) << 6,
+                      tfsf_inc_at(ax, side, slot, s->NZ) + cell[2], 0};
+      int& at = inc_at[x.dst];
+      if (at < 0) {
+        at = (int)s->incs.size();
+        s->incs.push_back(x);
+      } else {
+        const TfsfInc& y = s->incs[at];
+        if (y.dp != x.dp || y.idx != x.idx || y.meta != x.meta) s->inc_ok = false;
+      }
+    }
   }
   const size_t m = ent.size();
   out.n = (int)m;
@@ -569,6 +596,28 @@ static fdtd_status build_tfsf_table(fdtd_sim* s, const ShellCells& sh, int efiel
   out.ent = dent;
   out.term = dterm;
   return FDTD_OK;
+}
+
+template <typename T>
+static fdtd_status fuse_tfsf(fdtd_sim* s);
+
+// Below this many cells the passes apply the TFSF corrections (FDTD_TFSF=0 / 1:
+// never / always).  In the passes they cost registers and instructions in
+// proportion to the grid, in a launch of their own a launch and the faces' cells:
+// a step with the launch against without, us, FP32 64^3 10.3 / 9.0, 96^3 20.1 /
+// 18.7, 160x144x176 72.1 / 69.3, 256^3 272 / 267, 384x384x256 563 / 568; FP64
+// (half the cells a thread) 97x89x93 27.1 / 27.0, 256^3 524 / 531.
+static size_t fuse_tfsf_below(bool fp64) {
+  if (const char* e = std::getenv("FDTD_TFSF")) return e[0] == '0' ? 0 : (size_t)-1;
+  return fp64 ? (size_t)1 << 20 : (size_t)25000000;
+}
+
+// The direct passes (flat.cuh) run unless a knob of the staged ones is set, or
+// the grid is beyond their 32-bit cell offsets.
+static bool direct_passes(const fdtd_sim* s) {
+  const char* force = std::getenv("FDTD_PASS");
+  const bool knobs = (force && std::strncmp(force, "flat:", 5)) || std::getenv("FDTD_TMA") || std::getenv("FDTD_PDL");
+  return !knobs && s->ncell < ((size_t)1 << 31);
 }
 
 static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out, bool tune = true) {
@@ -820,6 +869,15 @@ static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out,
   CUDA_TRY(cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming));
   CUDA_TRY(cudaEventCreateWithFlags(&s->join_ev, cudaEventDisableTiming));
   CUDA_TRY(cudaDeviceSynchronize());
+  // The passes apply the TFSF corrections themselves where each depends on its
+  // face, component and z index alone (normal incidence): the line step then
+  // evaluates a few hundred increments a step.  Oblique incidence has nearly as
+  // many distinct corrections as face cells and keeps the TFSF launch.
+  s->fused_tfsf = direct_passes(s.get()) && s->inc_ok && tune && s->ncell < fuse_tfsf_below(s->fp64);
+  if (s->fused_tfsf) {
+    st = s->fp64 ? fuse_tfsf<double>(s.get()) : fuse_tfsf<float>(s.get());
+    if (st != FDTD_OK) return st;
+  }
   st = s->fp64 ? tune_passes<double>(s.get(), tune) : tune_passes<float>(s.get(), tune);
   if (st != FDTD_OK) return st;
   *out = s.release();
@@ -877,6 +935,26 @@ template <>
 MetalView<float>& mview<float>(fdtd_sim* s) { return s->mf; }
 template <>
 MetalView<double>& mview<double>(fdtd_sim* s) { return s->md; }
+
+// The increment arrays of the passes and the line step's list (their values
+// are state: the H launch of a step reads what the line step before it wrote).
+template <typename T>
+static fdtd_status fuse_tfsf(fdtd_sim* s) {
+  SimView<T>& v = view<T>(s);
+  T *h, *e;
+  TfsfInc* list;
+  CUDA_TRY(s->alloc(&h, (size_t)2 * 12 * s->NZ, true));
+  CUDA_TRY(s->alloc(&e, (size_t)12 * s->NZ, true));
+  CUDA_TRY(s->alloc(&list, s->incs.size()));
+  if (!s->incs.empty())
+    CUDA_TRY(cudaMemcpy(list, s->incs.data(), s->incs.size() * sizeof(TfsfInc), cudaMemcpyHostToDevice));
+  v.incH = h;
+  v.incE = e;
+  s->line.inc = list;
+  s->line.ninc = (int)s->incs.size();
+  s->line.nz = s->NZ;
+  return FDTD_OK;
+}
 
 template <typename T, int TY, int S>
 static size_t staged_smem() {
@@ -1082,19 +1160,53 @@ static void launch_ex(bool pdl, void (*kern)(P...), dim3 g, dim3 blk, size_t sme
 }
 
 // One launch of a direct pass (flat.cuh): kz planes per thread, one block per
-// kFlatThreads vectors and kz planes.  The H pass has a form whose plane loop
-// is unrolled by 8 (H reads E of plane k + 1, so the next plane's loads only
-// start early when the unrolled body hoists them: 256^3 FP32 119.7 us against
-// 136.8 rolled at kz = 8, 384 x 384 x 256 253.6 against 288.4); the E pass
-// reads plane k - 1, carried in registers, and is faster rolled (124.3 us
-// against 177.2).
+// kFlatThreads vectors and kz planes; ring: the planes copied ahead.
+// line: the launch carries the line's step (H) too; cells: and the dispersive
+// cells' share of it (the hydrodynamic currents in the H launch, the E updates
+// in the E launch).
 template <typename T, bool EPASS>
-static void launch_flat(fdtd_sim* s, int kz, int unroll, cudaStream_t st, bool pdl) {
-  const unsigned nv = (unsigned)(s->plane / Vec<T>::N), nbx = (nv + kFlatThreads - 1) / kFlatThreads;
-  const dim3 g(nbx * (unsigned)((s->NZ + kz - 1) / kz)), blk(kFlatThreads);
-  if (EPASS) launch_ex(pdl, e_flat<T, 1>, g, blk, 0, st, view<T>(s), nbx, kz);
-  else if (unroll == 8) launch_ex(pdl, h_flat<T, 8>, g, blk, 0, st, view<T>(s), nbx, kz);
-  else launch_ex(pdl, h_flat<T, 1>, g, blk, 0, st, view<T>(s), nbx, kz);
+static void launch_flat(fdtd_sim* s, int kz, int ring, cudaStream_t st, bool line = false, bool cells = false) {
+  const unsigned nv = (unsigned)(s->plane / Vec<T>::N), ntot = (unsigned)(s->nmetal[0] + s->nmetal[1] + s->nmetal[2]);
+  const bool hydro = s->su.hydro != 0;
+  FlatGrid g{(nv + kFlatThreads - 1) / kFlatThreads, 0, kz, line ? 1 : 0};
+  if (cells && (EPASS || hydro)) g.nrole = (ntot + kFlatThreads - 1) / kFlatThreads;
+  const dim3 grid(g.nbx * (unsigned)((s->NZ + kz - 1) / kz) + g.nrole + g.line), blk(kFlatThreads);
+  const SimView<T>& v = view<T>(s);
+  const MetalView<T>& m = mview<T>(s);
+  const size_t smem = ring ? kFlatRingBytes : 0;
+  const bool tfsf = s->fused_tfsf;
+#define FDTD_FLAT_E(KIND)                                                                                     \
+  (ring ? tfsf ? launch_ex(false, e_flat<T, true, true, KIND>, grid, blk, smem, st, v, m, g)                    \
+               : launch_ex(false, e_flat<T, true, false, KIND>, grid, blk, smem, st, v, m, g)                   \
+        : tfsf ? launch_ex(false, e_flat<T, false, true, KIND>, grid, blk, smem, st, v, m, g)                   \
+               : launch_ex(false, e_flat<T, false, false, KIND>, grid, blk, smem, st, v, m, g))
+#define FDTD_FLAT_H(HYDRO)                                                                                    \
+  (ring ? tfsf ? launch_ex(false, h_flat<T, true, true, HYDRO>, grid, blk, smem, st, v, m, s->line, s->probe_id, g)   \
+               : launch_ex(false, h_flat<T, true, false, HYDRO>, grid, blk, smem, st, v, m, s->line, s->probe_id, g)  \
+        : tfsf ? launch_ex(false, h_flat<T, false, true, HYDRO>, grid, blk, smem, st, v, m, s->line, s->probe_id, g)  \
+               : launch_ex(false, h_flat<T, false, false, HYDRO>, grid, blk, smem, st, v, m, s->line, s->probe_id, g))
+  if (EPASS) {
+    if (!g.nrole) FDTD_FLAT_E(0);
+    else if (!hydro) FDTD_FLAT_E(1);
+    else FDTD_FLAT_E(2);
+  } else {
+    if (g.nrole) FDTD_FLAT_H(true);
+    else FDTD_FLAT_H(false);
+  }
+#undef FDTD_FLAT_E
+#undef FDTD_FLAT_H
+}
+// The ring takes more than 48 KB of dynamic shared memory.
+template <typename T, bool TFSF>
+static cudaError_t flat_attributes() {
+  const void* k[5] = {(const void*)h_flat<T, true, TFSF, false>, (const void*)h_flat<T, true, TFSF, true>,
+                      (const void*)e_flat<T, true, TFSF, 0>, (const void*)e_flat<T, true, TFSF, 1>,
+                      (const void*)e_flat<T, true, TFSF, 2>};
+  for (const void* p : k) {
+    const cudaError_t e = cudaFuncSetAttribute(p, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatRingBytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // Launches one pass as its interior box (PML-free) and its edge table so
@@ -1107,7 +1219,7 @@ static void launch_flat(fdtd_sim* s, int kz, int unroll, cudaStream_t st, bool p
 template <typename T, bool EPASS>
 static int launch_pass_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st, bool chained = false) {
   if (c.kz) {
-    launch_flat<T, EPASS>(s, c.kz, c.unroll, st, chained);
+    launch_flat<T, EPASS>(s, c.kz, c.ring, st);
     return 1;
   }
   const fdtd_sim::TileSet& ts = tiles(s, c);
@@ -1159,15 +1271,17 @@ static int launch_e_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st
 // fastest.  Shapes: minimum CTAs per SM (register cap) x tile height x
 // z-chunk.  FDTD_TUNE=0 keeps the defaults.
 
-// The direct passes: planes per thread of each pass.  More planes per thread
-// re-read less (the k +- 1 plane is carried) but leave fewer blocks, so small
-// grids want few and wave quantisation decides in between (96^3: 3 planes 8.3
-// us, 2 or 4 planes 10.3 us; 256^3: 8 planes): timed on the zero state like the
-// staged shapes.  Untimed (FDTD_TUNE=0, batch members, under 2^18 cells) the
-// most planes, up to 8, that leave two blocks a multiprocessor.
-// FDTD_PASS=flat:KZ[:UNROLL] fixes them.
+// The direct passes: planes per thread of each pass, and whether they are copied
+// ahead.  More planes per thread re-read less (the k +- 1 plane is carried) but
+// leave fewer blocks, so small grids want few and wave quantisation decides in
+// between: timed on the zero state like the staged shapes.  Untimed (FDTD_TUNE=0,
+// batch members, under 2^18 cells) the most planes, up to 8, that leave two
+// blocks a multiprocessor, copied ahead from 4 planes on.
+// FDTD_PASS=flat:KZ[:RING] fixes them.
 template <typename T>
 static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force) {
+  if (s->fused_tfsf) CUDA_TRY((flat_attributes<T, true>()));
+  else CUDA_TRY((flat_attributes<T, false>()));
   fdtd_sim::PassCfg def;
   def.staged = 0;
   def.pdl = 1;
@@ -1176,49 +1290,78 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
   def.kz = 1;
   while (def.kz < 8 && nbx * ((s->NZ + 2 * def.kz - 1) / (2 * def.kz)) >= 2 * sms) def.kz *= 2;
-  def.unroll = def.kz == 8 ? 8 : 1;
+  def.ring = def.kz >= 4;
   if (force) {
-    if (std::sscanf(force, "flat:%d:%d", &def.kz, &def.unroll) < 1 || def.kz < 1 ||
-        (def.unroll != 1 && def.unroll != 8))
+    if (std::sscanf(force, "flat:%d:%d", &def.kz, &def.ring) < 1 || def.kz < 1 || def.ring < 0 || def.ring > 1)
       return fail(FDTD_ERR_INVALID, "FDTD_PASS names a pass variant that is not built");
   }
-  def.kchunk = def.kz;
-  def.stages = def.estages = def.unroll;
+  auto report = [](fdtd_sim::PassCfg& c) {
+    c.kchunk = c.kz;
+    c.stages = c.estages = c.ring ? kFlatRing : 1;
+  };
+  report(def);
   s->hcfg = s->ecfg = def;
   s->tuned = true;
   const char* env = std::getenv("FDTD_TUNE");
   if (!time_variants || (env && env[0] == '0') || force || s->ncell < (size_t)(1 << 18)) return FDTD_OK;
   const char* venv = std::getenv("FDTD_TUNE_VERBOSE");
   const bool verbose = venv && venv[0] == '1';
+  // each candidate as a graph of launches, as the steps run it: small passes are
+  // shorter than a launch from the host
+  // (a ring pays from grids beyond L2 on, and with several planes to run ahead)
+  const bool big = s->ncell >= (size_t)(1 << 21);
+  std::vector<int> kzs = {4, 6, 8};
+  if (big) kzs.insert(kzs.end(), {12, 16, 32});
+  else kzs.insert(kzs.end(), {1, 2, 3});
+  for (int waves = 1; waves <= 2; waves++) {  // the fewest planes that fill the GPU's block slots this many times
+    const long long per = 2LL * sms * waves / nbx;
+    if (per > 0) kzs.push_back((int)((s->NZ + per - 1) / per));
+  }
+  std::sort(kzs.begin(), kzs.end());
+  kzs.erase(std::unique(kzs.begin(), kzs.end()), kzs.end());
+  const int reps = s->ncell > (size_t)(1 << 23) ? 4 : 6;
   cudaEvent_t a, b;
+  cudaStream_t st;
   CUDA_TRY(cudaEventCreate(&a));
   CUDA_TRY(cudaEventCreate(&b));
-  for (int pass = 0; pass < 2; pass++) {
+  CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  cudaError_t err = cudaSuccess;
+  for (int pass = 0; pass < 2 && err == cudaSuccess; pass++) {
     fdtd_sim::PassCfg& best = pass == 0 ? s->hcfg : s->ecfg;
     float best_ms = 1e30f;
-    for (int kz : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    for (int kz : kzs) {
       if (kz > s->NZ) continue;
-      for (int unroll : {1, 8}) {
-        if (unroll == 8 && (pass == 1 || kz < 8)) continue;
+      for (int ring = 0; ring < 2; ring++) {
+        if (ring ? !big || kz < 4 : big && (kz == 6 || kz == 12 || kz > 16)) continue;
         fdtd_sim::PassCfg c = def;
-        c.kz = c.kchunk = kz;
-        c.unroll = c.stages = c.estages = unroll;
-        auto go = [&]() {
-          if (pass == 0) launch_flat<T, false>(s, kz, unroll, 0, false);
-          else launch_flat<T, true>(s, kz, unroll, 0, false);
-        };
-        go();
-        go();
-        CUDA_TRY(cudaEventRecord(a));
-        for (int r = 0; r < 10; r++) go();
-        CUDA_TRY(cudaEventRecord(b));
-        CUDA_TRY(cudaEventSynchronize(b));
-        float ms;
-        CUDA_TRY(cudaEventElapsedTime(&ms, a, b));
-        c.ms = ms / 10;
+        c.kz = kz;
+        c.ring = ring;
+        report(c);
+        cudaGraph_t g = nullptr;
+        cudaGraphExec_t x = nullptr;
+        err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+        if (err != cudaSuccess) break;
+        for (int r = 0; r < reps; r++) {
+          if (pass == 0) launch_flat<T, false>(s, kz, ring, st);
+          else launch_flat<T, true>(s, kz, ring, st);
+        }
+        err = cudaStreamEndCapture(st, &g);
+        if (err == cudaSuccess) err = cudaGraphInstantiate(&x, g, 0);
+        if (g) cudaGraphDestroy(g);
+        float ms = 0.f;
+        for (int r = 0; r < 2 && err == cudaSuccess; r++) {  // the first run warms up
+          cudaEventRecord(a, st);
+          err = cudaGraphLaunch(x, st);
+          cudaEventRecord(b, st);
+          if (err == cudaSuccess) err = cudaEventSynchronize(b);
+          if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, a, b);
+        }
+        if (x) cudaGraphExecDestroy(x);
+        if (err != cudaSuccess) break;
+        c.ms = ms / reps;
         if (verbose)
-          std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread (unrolled by %d): %.4f ms\n",
-                       pass == 0 ? "H" : "E", kz, unroll, c.ms);
+          std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread%s: %.4f ms\n", pass == 0 ? "H" : "E", kz,
+                       ring ? ", copied ahead" : "", c.ms);
         if (c.ms < best_ms) {
           best_ms = c.ms;
           best = c;
@@ -1228,6 +1371,8 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
+  cudaStreamDestroy(st);
+  CUDA_TRY(err);
   CUDA_TRY(cudaGetLastError());
   return FDTD_OK;
 }
@@ -1235,13 +1380,7 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
 template <typename T>
 static fdtd_status tune_passes(fdtd_sim* s, bool time_variants) {
   CUDA_TRY(cudaFuncSetAttribute(dft_contract<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_smem_bytes<T>()));
-  // The direct passes run unless a knob of the staged ones is set, or the
-  // grid is beyond their 32-bit cell offsets.
-  {
-    const char* force = std::getenv("FDTD_PASS");
-    const bool knobs = (force && std::strncmp(force, "flat:", 5)) || std::getenv("FDTD_TMA") || std::getenv("FDTD_PDL");
-    if (!knobs && s->ncell < ((size_t)1 << 31)) return tune_flat<T>(s, time_variants, force);
-  }
+  if (direct_passes(s)) return tune_flat<T>(s, time_variants, std::getenv("FDTD_PASS"));
   staged_attributes<T>();
   // defaults; FDTD_PASS=staged:TY:MINB:KCHUNK[:STAGES] forces a variant,
   // FDTD_TUNE=0 skips the timing, small grids are not worth timing
@@ -1402,7 +1541,7 @@ static fdtd_status tune_passes(fdtd_sim* s, bool time_variants) {
 template <typename T>
 static void launch_h(fdtd_sim* s, cudaStream_t st) {
   s->kernels += launch_h_cfg<T>(s, s->hcfg, st);
-  const int nf = s->tf_h.n;
+  const int nf = s->fused_tfsf ? 0 : s->tf_h.n;
   if (nf > 0) {
     tfsf_h_apply<T><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(view<T>(s), s->tf_h, s->line);
     s->kernels++;
@@ -1420,11 +1559,22 @@ static void launch_e_pass(fdtd_sim* s, cudaStream_t st);
 
 template <typename T>
 static void launch_e(fdtd_sim* s, cudaStream_t st) {
-  const int nf = s->tf_e.n;
+  const int nf = s->fused_tfsf ? 0 : s->tf_e.n;
   // E half of CORRECT_* before the update (main.cu:2798-2813)
   if (nf > 0) {
     tfsf_e_apply<T><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(view<T>(s), s->tf_e);
     s->kernels++;
+  }
+  if (s->ecfg.kz) {
+    // the fused step computes the hydrodynamic currents in its H launch
+    const int ntot = s->nmetal[0] + s->nmetal[1] + s->nmetal[2];
+    if (s->su.hydro && ntot > 0) {
+      hydro_p<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
+      s->kernels++;
+    }
+    launch_flat<T, true>(s, s->ecfg.kz, s->ecfg.ring, st, false, true);
+    s->kernels++;
+    return;
   }
   launch_e_pass<T>(s, st);
 }
@@ -1432,9 +1582,10 @@ static void launch_e(fdtd_sim* s, cudaStream_t st) {
 // The fused step's TFSF: both halves in one launch, after the line step.
 template <typename T>
 static void launch_tfsf(fdtd_sim* s, cudaStream_t st) {
-  const int nf = s->tf_h.n + s->tf_e.n;
+  const int nf = s->fused_tfsf ? 0 : s->tf_h.n + s->tf_e.n;
   if (nf > 0) {
-    tfsf_apply<T><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(view<T>(s), s->tf_h, s->tf_e, s->line);
+    launch_ex(false, tfsf_apply<T>, dim3((unsigned)((nf + 255) / 256)), dim3(256), 0, st, view<T>(s), s->tf_h, s->tf_e,
+              s->line);
     s->kernels++;
   }
 }
@@ -1467,9 +1618,9 @@ static void launch_e_pass(fdtd_sim* s, cudaStream_t st) {
   }
 }
 
-// The dispersive cells' kernels; chained: the hydrodynamic phases after the
-// first carry a programmatic dependency on the phase before (they wait for
-// it at their start).
+// The dispersive cells' kernels (staged passes); chained: the hydrodynamic E
+// update carries a programmatic dependency on the currents' launch (it waits
+// for it at its start).
 template <typename T>
 static void launch_metal(fdtd_sim* s, cudaStream_t st, bool chained) {
   const int ntot = s->nmetal[0] + s->nmetal[1] + s->nmetal[2];
@@ -1478,19 +1629,11 @@ static void launch_metal(fdtd_sim* s, cudaStream_t st, bool chained) {
     metal_e<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
     s->kernels++;
   } else {
-    // UpdateHydroP* of every cell fused with the Ex update, then Ey, Ez
-    hydro_p_ex<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
-    s->kernels++;
-    if (s->nmetal[1] > 0) {
-      launch_ex(chained, hydro_e<T, 1>, dim3((s->nmetal[1] + 127) / 128), dim3(128), 0, st, view<T>(s), mview<T>(s),
-                (const DevClock*)s->clk);
-      s->kernels++;
-    }
-    if (s->nmetal[2] > 0) {
-      launch_ex(chained, hydro_e<T, 2>, dim3((s->nmetal[2] + 127) / 128), dim3(128), 0, st, view<T>(s), mview<T>(s),
-                (const DevClock*)s->clk);
-      s->kernels++;
-    }
+    // UpdateHydroP* of every cell, then the E updates
+    hydro_p<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
+    launch_ex(chained, hydro_e<T>, dim3((ntot + 127) / 128), dim3(128), 0, st, view<T>(s), mview<T>(s),
+              (const DevClock*)s->clk);
+    s->kernels += 2;
   }
 }
 template <typename T>
@@ -1498,7 +1641,7 @@ static void launch_sample(fdtd_sim* s, cudaStream_t st) {
   int maxn = 0;
   for (int f = 0; f < s->dft.nfaces; f++) maxn = std::max(maxn, s->dft.face[f].na * s->dft.face[f].nb);
   dim3 g((maxn + 255) / 256, s->dft.nfaces);
-  dft_sample<T><<<g, 256, 0, st>>>(view<T>(s), s->dft, (T*)s->ring, s->clk);
+  launch_ex(false, dft_sample<T>, g, dim3(256), 0, st, view<T>(s), s->dft, (T*)s->ring, (const DevClock*)s->clk);
   s->kernels++;
 }
 // The contraction of the clock's job (dft_job_*): phasors, then the FP64
@@ -1542,6 +1685,14 @@ static void sample_and_contract(fdtd_sim* s, cudaStream_t st) {
   if (s->host_nsamp == kRingSlots) s->host_nsamp = 0;
 }
 
+template <typename T>
+static void launch_snap(fdtd_sim* s, cudaStream_t st) {
+  const int n = std::max(s->snap.rows * s->snap.cols, std::max(s->snap.aux_len, s->snap.line_len));
+  launch_ex(false, snap_gather<T>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, view<T>(s), mview<T>(s), s->line,
+            s->snap);
+  s->kernels++;
+}
+
 // One full step.  The 1-D line step runs beside the H pass (on the second
 // side stream, or before it on the same stream with the pass launched as a
 // programmatic dependent when the pass's launches run on one stream): it
@@ -1555,6 +1706,22 @@ static void sample_and_contract(fdtd_sim* s, cudaStream_t st) {
 template <typename T>
 static void enqueue_step(fdtd_sim* s, cudaStream_t st) {
   dft_period_begin<T>(s, st);
+  if (s->hcfg.kz) {
+    // two launches a step: H with the line and the hydrodynamic currents, E with
+    // the dispersive cells (and the TFSF launch between them where the passes do
+    // not apply it).  Plain launches: with programmatic dependencies the next
+    // launch's blocks, resident early, take the slots that free first and the
+    // single-wave passes end up unevenly spread (97 x 89 x 93 FP64 33.0 us a step
+    // against 26.5, 96^3 20.8 against 18.3, 256^3 FP32 250.3 against 246.2).
+    launch_flat<T, false>(s, s->hcfg.kz, s->hcfg.ring, st, true, true);
+    launch_tfsf<T>(s, st);
+    launch_flat<T, true>(s, s->ecfg.kz, s->ecfg.ring, st, false, true);
+    s->kernels += 2;
+    if (s->line.dft_every > 0 && s->t % s->line.dft_every == 0) sample_and_contract<T>(s, st);
+    if (s->snap_on) launch_snap<T>(s, st);
+    s->t++;
+    return;
+  }
   if (s->hcfg.pdl) {
     // one stream, without a fork: the line, then the H pass with a
     // programmatic dependency on it (the pass starts at once and waits for
@@ -1572,11 +1739,7 @@ static void enqueue_step(fdtd_sim* s, cudaStream_t st) {
   launch_tfsf<T>(s, st);
   launch_e_pass<T>(s, st);
   if (s->line.dft_every > 0 && s->t % s->line.dft_every == 0) sample_and_contract<T>(s, st);
-  if (s->snap_on) {
-    const int n = std::max(s->snap.rows * s->snap.cols, std::max(s->snap.aux_len, s->snap.line_len));
-    snap_gather<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(view<T>(s), mview<T>(s), s->line, s->snap);
-    s->kernels++;
-  }
+  if (s->snap_on) launch_snap<T>(s, st);
   s->t++;
 }
 

@@ -38,6 +38,8 @@ struct DevClock {
   int base;       // first slot of the half being filled (0 or kRingSlots)
   int cstart;     // samples of that half a flush has already contracted
   int job_off, job_n, job_reset;
+  int th;         // the step as the H launch of the fused step reads it: t moves on inside that launch
+                  // (its line block), th follows in the E launch; equal between steps
   int samp_t[2 * kRingSlots];
 };
 
@@ -90,11 +92,21 @@ struct SimView {
                         // line's E is double-buffered and passed per launch
   int* nonfinite;
   const SimView* self;  // a copy of this view in device memory (cold paths)
-  // this step's TFSF increments of the H and the E faces (flat.cuh), null when
-  // the TFSF launch applies the corrections
-  const T* incH;
-  const T* incE;
+  // the step's TFSF increments of the H faces (two buffers, by step parity)
+  // and the E faces (flat.cuh), null when the TFSF launch applies the
+  // corrections
+  T* incH;
+  T* incE;
+  DevClock* clk;
   int periodic;         // 1: x and y wrap around (every x and y index is updated)
+};
+
+// One TFSF increment of the step: the incident value between line points idx
+// and idx + 1, weight dp on the right one, as a correction of face entry dst.
+// meta = (sign > 0) | axis << 1 | component << 3 | (E half) << 5 | class << 6
+struct TfsfInc {
+  double dp;
+  int idx, meta, dst, pad;
 };
 
 // Dispersive (Drude + 2 critical points, optionally hydrodynamic) cells.
@@ -110,7 +122,7 @@ struct MetalView {
   T* en[3]; T* en1[3];
   double* cpn[3][2]; double* cpn1[3][2];
   double* pd[3][3];     // Drude current ring (n, n-1, new) indexed by step
-  double* nd[3][2];     // hydro density ring
+  double* nd[3][3];     // hydro density ring, the same indexing
   const float* rho[3];  // design blend per slot (null: plain metal coefficients)
   double vac;           // vacuum C_E = C_E_1 = ep0, the rho = 0 end of the blend
   // forward record for the adjoint (null = off): per step t the row

@@ -52,6 +52,46 @@ __device__ __forceinline__ Vec<T> zerov() {
 
 constexpr int kFlatThreads = 256;
 
+// A thread's own vectors of the planes to come, copied into shared memory
+// asynchronously S - 1 planes ahead.  No other thread reads them, so the ring
+// needs no barrier: it stands in for registers that would hold the loads of
+// several planes.
+constexpr int kFlatRing = 4;
+constexpr int kFlatRingBytes = kFlatRing * 6 * kFlatThreads * 16;
+template <typename T>
+struct FlatRing {
+  unsigned base;
+  __device__ __forceinline__ void init() {
+    extern __shared__ __align__(16) unsigned char flat_smem[];
+    base = (unsigned)__cvta_generic_to_shared(flat_smem) + threadIdx.x * 16u;
+  }
+  __device__ __forceinline__ void issue(int st, int a, const T* p) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + (unsigned)((st * 6 + a) * kFlatThreads * 16)),
+                 "l"(p));
+  }
+  __device__ __forceinline__ Vec<float> get(int st, int a, float) {
+    Vec<float> r;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])
+                 : "r"(base + (unsigned)((st * 6 + a) * kFlatThreads * 16)));
+    return r;
+  }
+  __device__ __forceinline__ Vec<double> get(int st, int a, double) {
+    Vec<double> r;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n"
+                 : "=d"(r.v[0]), "=d"(r.v[1])
+                 : "r"(base + (unsigned)((st * 6 + a) * kFlatThreads * 16)));
+    return r;
+  }
+  __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+  __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(kFlatRing - 2) : "memory"); }
+};
+// a line another plane of this thread will need, into L2
+template <typename T>
+__device__ __forceinline__ void flat_touch(const T* p) {
+  asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+
 // CPML of one vector and one axis: psi <- b psi + c diff / d per lane, and
 // the field += sg coef psi; w = lanes that are updated (the others keep psi).
 template <typename T>
@@ -95,82 +135,32 @@ __device__ __forceinline__ void add_lanes(Vec<T>& v, unsigned m, T x) {
     if ((m >> l) & 1) v.v[l] += x;
 }
 
-// The step's TFSF increments on the faces (CORRECT_X/Y/Z, main.cu:369-758) of
-// a plane wave along z: per face (axis, side) and tangential component (slot
-// 0 = the axis after the normal, 1 = the one after that) one value per z
-// index, the sign included; zero where the incident field has no such
-// component.  line_flat fills them from the 1D line (TfsfInc below).
-__host__ __device__ __forceinline__ int tfsf_inc_at(int axis, int side, int slot, int NZ) {
-  return ((axis * 2 + side) * 2 + slot) * NZ;
-}
+// The step's TFSF increments (tfsf_inc_at, kernels.cuh) in a pass.  The wave
+// runs along z, so that on the x and y faces only the z component takes one: a
+// lane of the vector on an x face and the lanes of a row on a y face.  Which,
+// and on which side, is fixed along a thread's planes and kept in one word:
+// bits 0-3 the x face's lane, 4-7 the y face's lanes, 8 / 9 their sides
+// (finding them per plane cost the 256^3 H pass 8 us of 121, as did keeping
+// masks and pointers apart, which spills).  The z faces are two planes of the
+// grid.  half = 0: hz, half-open in x and y; half = 1: ez, closed in x and y.
 template <typename T>
-__device__ __forceinline__ void h_flat_tfsf(const SimView<T>& s, int i0, int j, int k, Vec<T>& hx, Vec<T>& hy,
-                                            Vec<T>& hz) {
+__device__ __forceinline__ unsigned flat_faces(const SimView<T>& s, int half, int i0, int j) {
   constexpr int N = Vec<T>::N;
-  const int NX = s.NX, NY = s.NY, NZ = s.NZ, Tx = s.tf.Tx, Ty = s.tf.Ty, Tz = s.tf.Tz;
-  const T* inc = s.incH + k;
-  const bool kin = k >= Tz && k < NZ - Tz, kon = k >= Tz;       // half-open, closed (k <= NZ - Tz holds)
-  const bool jin = j >= Ty && j < NY - Ty, jon = j >= Ty && j <= NY - Ty;
-#pragma unroll
-  for (int side = 0; side < 2; side++) {
-    const int fx = side ? NX - Tx : Tx - 1, fy = side ? NY - Ty : Ty - 1, fz = side ? NZ - Tz : Tz - 1;
-    if (fx >= i0 && fx < i0 + N) {
-      const unsigned m = 1u << (fx - i0);
-      if (jon && kin) add_lanes(hy, m, inc[tfsf_inc_at(0, side, 0, NZ)]);
-      if (jin && kon) add_lanes(hz, m, inc[tfsf_inc_at(0, side, 1, NZ)]);
-    }
-    if (j == fy) {
-      if (kon) add_lanes(hz, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(1, side, 0, NZ)]);
-      if (kin) add_lanes(hx, lanes_in<N>(i0, Tx, NX - Tx + 1), inc[tfsf_inc_at(1, side, 1, NZ)]);
-    }
-    if (k == fz) {
-      if (jin) add_lanes(hx, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), inc[tfsf_inc_at(2, side, 0, NZ)]);
-      if (jon) add_lanes(hy, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(2, side, 1, NZ)]);
-    }
+  const int NX = s.NX, NY = s.NY, Tx = s.tf.Tx, Ty = s.tf.Ty, off = half ? 0 : 1;
+  unsigned m = 0;
+  if (j >= Ty && j < NY - Ty + half) {
+    const int lo = Tx - off - i0, hi = NX - Tx - i0;
+    if (lo >= 0 && lo < N) m |= 1u << lo;
+    if (hi >= 0 && hi < N) m |= 1u << hi | 256u;
   }
+  if (j == Ty - off || j == NY - Ty) m |= lanes_in<N>(i0, Tx, NX - Tx + half) << 4 | (j == NY - Ty ? 512u : 0u);
+  return m;
 }
-// The E half, added to E before its update; axis by axis (an edge cell takes
-// two corrections, in the order X, Y, Z).
-template <typename T>
-__device__ __forceinline__ void e_flat_tfsf(const SimView<T>& s, int i0, int j, int k, Vec<T>& ex, Vec<T>& ey,
-                                            Vec<T>& ez) {
-  constexpr int N = Vec<T>::N;
-  const int NX = s.NX, NY = s.NY, NZ = s.NZ, Tx = s.tf.Tx, Ty = s.tf.Ty, Tz = s.tf.Tz;
-  const T* inc = s.incE + k;
-  const bool kin = k < NZ - Tz;  // Tz <= k <= NZ - Tz holds
-  const bool jin = j >= Ty && j < NY - Ty, jon = j >= Ty && j <= NY - Ty;
-#pragma unroll
-  for (int side = 0; side < 2; side++) {
-    const int fx = side ? NX - Tx : Tx;
-    if (fx >= i0 && fx < i0 + N) {
-      const unsigned m = 1u << (fx - i0);
-      if (jin) add_lanes(ey, m, inc[tfsf_inc_at(0, side, 0, NZ)]);
-      if (jon && kin) add_lanes(ez, m, inc[tfsf_inc_at(0, side, 1, NZ)]);
-    }
-  }
-#pragma unroll
-  for (int side = 0; side < 2; side++) {
-    const int fy = side ? NY - Ty : Ty;
-    if (j == fy) {
-      if (kin) add_lanes(ez, lanes_in<N>(i0, Tx, NX - Tx + 1), inc[tfsf_inc_at(1, side, 0, NZ)]);
-      add_lanes(ex, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(1, side, 1, NZ)]);
-    }
-  }
-#pragma unroll
-  for (int side = 0; side < 2; side++) {
-    const int fz = side ? NZ - Tz : Tz;
-    if (k == fz) {
-      if (jon) add_lanes(ex, lanes_in<N>(i0, Tx, NX - Tx), inc[tfsf_inc_at(2, side, 0, NZ)]);
-      if (jin) add_lanes(ey, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), inc[tfsf_inc_at(2, side, 1, NZ)]);
-    }
-  }
-}
-
 // H pass (UPDATE_hx/hy/hz, main.cu:762-1044) of the vector vq of the plane,
 // planes k0 .. k0+KZ-1.  Same arithmetic and order per cell as h_pass_tile
 // (staged.cuh); the H half of CORRECT_X/Y/Z is added to the updated value
 // from the step's increments (incH) when the view carries them.
-template <typename T, int U>
+template <typename T, bool RING, bool TFSF>
 __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, int k0, int kz) {
   constexpr int N = Vec<T>::N;
   const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
@@ -192,48 +182,90 @@ __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, i
   // CPML slabs of this vector
   const int xs = s.cp[0].Nc <= 0 ? -1 : i0 < s.cp[0].Wn ? i0 : (i0 + N > s.cp[0].fb ? i0 - s.cp[0].fb + s.cp[0].Wn : -1);
   const bool yfar = j >= s.cp[1].F;
-  const int ys = s.cp[1].Nc <= 0 ? -1 : j < s.cp[1].Nc ? j : (yfar && j < NY - 1 ? j - s.cp[1].F : -1);
+  // (the far y slab follows the near one, NZ planes of Nc rows on)
+  const int ys = s.cp[1].Nc <= 0 ? -1 : j < s.cp[1].Nc ? j : (yfar && j < NY - 1 ? j - s.cp[1].F + NZ * s.cp[1].Nc : -1);
   const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
   // next vector's first value along x, from the next lane
   const bool edge = lane == 31 || i0 + N >= PX;
   const int ox = i0 + N < PX ? N : (per ? N - PX : 0);
-  const TfsfView& tf = s.tf;
-  const bool tfsf = s.incH != nullptr;
-  const unsigned b0 = (unsigned)k0 * plane + c0;
-  Vec<T> ex = ldgv(s.E[0] + b0), ey = ldgv(s.E[1] + b0);
+  const T* incH = TFSF && s.incH ? s.incH + (size_t)(s.clk->th & 1) * 12 * NZ : nullptr;
+  const unsigned face = incH ? flat_faces(s, 0, i0, j) : 0u;
+  // downwards: Ex and Ey of plane k + 1 come in registers, and the plane's own
+  // loads are all of plane k, with the +y row's just loaded by its own thread
   const int k1 = min(k0 + kz, NZ);
-#pragma unroll U
-  for (int k = k0; k < k1; k++) {
+  const unsigned b1 = (unsigned)min(k1, NZ - 1) * plane + c0;
+  Vec<T> exn = ldgv(s.E[0] + b1), eyn = ldgv(s.E[1] + b1);
+  FlatRing<T> ring;
+  int st = 0;
+  auto issue = [&](int stage, int k) {
+    if (k >= k0) {
+      const unsigned b = (unsigned)k * plane + c0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        ring.issue(stage, c, s.E[c] + b);
+        ring.issue(stage, 3 + c, s.H[c] + b);
+      }
+    }
+    ring.commit();
+  };
+  if (RING) {
+    ring.init();
+#pragma unroll
+    for (int q = 0; q < kFlatRing - 1; q++) issue(q, k1 - 1 - q);
+  }
+#pragma unroll 1
+  for (int k = k1 - 1; k >= k0; k--) {
     const unsigned b = (unsigned)k * plane + c0;
     const bool hask = k + 1 < NZ;
-    const unsigned bn = hask ? b + plane : b;
     // every load of the plane
-    const Vec<T> ez = ldgv(s.E[2] + b);
-    const Vec<T> exn = ldgv(s.E[0] + bn), eyn = ldgv(s.E[1] + bn);
     const Vec<T> exj = ldgv(s.E[0] + b + oj), ezj = ldgv(s.E[2] + b + oj);
-    Vec<T> hx = ldv(s.H[0] + b), hy = ldv(s.H[1] + b), hz = ldv(s.H[2] + b);
+    Vec<T> ex, ey, ez, hx, hy, hz;
+    if (!RING) {
+      ex = ldgv(s.E[0] + b); ey = ldgv(s.E[1] + b); ez = ldgv(s.E[2] + b);
+      hx = ldv(s.H[0] + b); hy = ldv(s.H[1] + b); hz = ldv(s.H[2] + b);
+    }
     T eyi = T(0), ezi = T(0);
     if (edge) { eyi = ldg(s.E[1] + b + ox); ezi = ldg(s.E[2] + b + ox); }
     const T ikz = ldg(s.cp[2].inv_khd + k);
-    T *px0 = nullptr, *px1 = nullptr, *py0 = nullptr, *py1 = nullptr, *pz0 = nullptr, *pz1 = nullptr;
+    unsigned ozo = 0, oxo = 0, oyo = 0;  // offsets in the psi arrays
     Vec<T> ox0, ox1, oy0, oy1, oz0, oz1;
     int zs = -1;
     if (hask && Ncz > 0) zs = k < Ncz ? k : (k >= Fz ? k - Fz + Ncz : -1);
     if (zs >= 0) {
-      const unsigned o = (unsigned)zs * plane + c0;
-      pz0 = s.psiH_N[0][1] + o; pz1 = s.psiH_N[1][0] + o;
-      oz0 = ldv(pz0); oz1 = ldv(pz1);
+      ozo = (unsigned)zs * plane + c0;
+      oz0 = ldv(s.psiH_N[0][1] + ozo); oz1 = ldv(s.psiH_N[1][0] + ozo);
     }
     if (xs >= 0 && hask) {
-      const unsigned o = ((unsigned)k * NY + j) * s.cp[0].W + xs;
-      px0 = s.psiH_N[1][1] + o; px1 = s.psiH_N[2][0] + o;
-      ox0 = ldv(px0); ox1 = ldv(px1);
+      oxo = ((unsigned)k * NY + j) * s.cp[0].W + xs;
+      ox0 = ldv(s.psiH_N[1][1] + oxo); ox1 = ldv(s.psiH_N[2][0] + oxo);
     }
     if (ys >= 0 && hask) {
-      const unsigned o = ((unsigned)k * s.cp[1].Nc + ys) * PX + i0;
-      py0 = (yfar ? s.psiH_F[0][0] : s.psiH_N[0][0]) + o;
-      py1 = (yfar ? s.psiH_F[2][1] : s.psiH_N[2][1]) + o;
-      oy0 = ldv(py0); oy1 = ldv(py1);
+      oyo = ((unsigned)k * s.cp[1].Nc + ys) * PX + i0;
+      oy0 = ldv(s.psiH_N[0][0] + oyo); oy1 = ldv(s.psiH_N[2][1] + oyo);
+    }
+    if (RING) {
+      if (k > k0) {  // the next plane's psi
+        if (xs >= 0) {
+          const unsigned o = ((unsigned)(k - 1) * NY + j) * s.cp[0].W + xs;
+          flat_touch(s.psiH_N[1][1] + o);
+          flat_touch(s.psiH_N[2][0] + o);
+        }
+        if (ys >= 0) {
+          const unsigned o = ((unsigned)(k - 1) * s.cp[1].Nc + ys) * PX + i0;
+          flat_touch(s.psiH_N[0][0] + o);
+          flat_touch(s.psiH_N[2][1] + o);
+        }
+      }
+      ring.wait();
+      issue(st == 0 ? kFlatRing - 1 : st - 1, k - (kFlatRing - 1));
+      ex = ring.get(st, 0, T(0)); ey = ring.get(st, 1, T(0)); ez = ring.get(st, 2, T(0));
+      hx = ring.get(st, 3, T(0)); hy = ring.get(st, 4, T(0)); hz = ring.get(st, 5, T(0));
+      st = st == kFlatRing - 1 ? 0 : st + 1;
+    }
+    T fx = T(0), fy = T(0);  // TFSF increments (loaded last: they wait for the clock)
+    if (TFSF && face && k >= s.tf.Tz && k <= NZ - s.tf.Tz) {
+      if (face & 15u) fx = incH[tfsf_inc_at(0, (face >> 8) & 1, 1, NZ) + k];
+      if (face & 240u) fy = incH[tfsf_inc_at(1, (face >> 9) & 1, 0, NZ) + k];
     }
     {
       const T a = __shfl_down_sync(0xFFFFFFFFu, ey.v[0], 1), c = __shfl_down_sync(0xFFFFFFFFu, ez.v[0], 1);
@@ -263,18 +295,18 @@ __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, i
     if (wp) {
       if (zs >= 0) {
         const T bz = ldg(s.cp[2].bh + k), cz = ldg(s.cp[2].ch + k);
-        psi_vec(pz0, oz0, &bz, &cz, false, s.cp[2].inv_d, dzy, vx, T(1), che, wp, true);
-        psi_vec(pz1, oz1, &bz, &cz, false, s.cp[2].inv_d, dzx, vy, T(-1), che, wp, true);
+        psi_vec(s.psiH_N[0][1] + ozo, oz0, &bz, &cz, false, s.cp[2].inv_d, dzy, vx, T(1), che, wp, true);
+        psi_vec(s.psiH_N[1][0] + ozo, oz1, &bz, &cz, false, s.cp[2].inv_d, dzx, vy, T(-1), che, wp, true);
       }
       if (xs >= 0 && hask) {
         const Vec<T> bx = ldgv(s.cp[0].bh + i0), cx = ldgv(s.cp[0].ch + i0);
-        psi_vec(px0, ox0, bx.v, cx.v, true, s.cp[0].inv_d, dxz, vy, T(1), che, wp, true);
-        psi_vec(px1, ox1, bx.v, cx.v, true, s.cp[0].inv_d, dxy, vz, T(-1), che, wp, true);
+        psi_vec(s.psiH_N[1][1] + oxo, ox0, bx.v, cx.v, true, s.cp[0].inv_d, dxz, vy, T(1), che, wp, true);
+        psi_vec(s.psiH_N[2][0] + oxo, ox1, bx.v, cx.v, true, s.cp[0].inv_d, dxy, vz, T(-1), che, wp, true);
       }
       if (ys >= 0 && hask) {
         const T by = ldg(s.cp[1].bh + j), cy = ldg(s.cp[1].ch + j);
-        psi_vec(py0, oy0, &by, &cy, false, s.cp[1].inv_d, dyz, vx, T(-1), che, wp, true);
-        psi_vec(py1, oy1, &by, &cy, false, s.cp[1].inv_d, dyx, vz, T(1), che, wp, true);
+        psi_vec(s.psiH_N[0][0] + oyo, oy0, &by, &cy, false, s.cp[1].inv_d, dyz, vx, T(-1), che, wp, true);
+        psi_vec(s.psiH_N[2][1] + oyo, oy1, &by, &cy, false, s.cp[1].inv_d, dyx, vz, T(1), che, wp, true);
       }
     }
 #pragma unroll
@@ -283,23 +315,60 @@ __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, i
       hx.v[l] = vx.v[l];
       if (on) { hy.v[l] = vy.v[l]; hz.v[l] = vz.v[l]; }
     }
-    if (tfsf && k >= tf.Tz - 1 && k <= NZ - tf.Tz) h_flat_tfsf(s, i0, j, k, hx, hy, hz);
+    // the H half of CORRECT_X/Y/Z
+    if (TFSF && face) {
+      add_lanes(hz, face & 15u, fx);
+      add_lanes(hz, (face >> 4) & 15u, fy);
+    }
+    if (TFSF && incH && (k == s.tf.Tz - 1 || k == NZ - s.tf.Tz)) {
+      const int side = k == NZ - s.tf.Tz, Tx = s.tf.Tx, Ty = s.tf.Ty;
+      if (j >= Ty && j < NY - Ty) add_lanes(hx, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), incH[tfsf_inc_at(2, side, 0, NZ) + k]);
+      if (j >= Ty && j <= NY - Ty) add_lanes(hy, lanes_in<N>(i0, Tx, NX - Tx), incH[tfsf_inc_at(2, side, 1, NZ) + k]);
+    }
     if (in) {
       if (hasy && hask) stv(s.H[0] + b, hx);
       if (hask) stv(s.H[1] + b, hy);
       if (hasy) stv(s.H[2] + b, hz);
     }
-    ex = exn;
-    ey = eyn;
+    exn = ex;
+    eyn = ey;
   }
 }
 
-template <typename T, int U>
-__global__ void __launch_bounds__(kFlatThreads, 2) h_flat(const __grid_constant__ SimView<T> s, unsigned nbx, int kz) {
-  pdl_launch_dependents();
-  const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
-  h_flat_cells<T, U>(s, xb * kFlatThreads + threadIdx.x, (int)kb * kz, kz);
-  pdl_wait();
+// Which blocks of a launch do what: block 0 the 1D line (H launches with
+// line = 1), the next nrole blocks the dispersive cells, the others the
+// grid's vectors, nbx blocks a group of kz planes.
+struct FlatGrid {
+  unsigned nbx, nrole;
+  int kz, line;
+};
+
+// The H launch of a step: the H pass, with it the 1D line's step (it reads E
+// at the probe cell, the line and the clock, and writes the line's other E
+// buffer, the line's H and the increments of the coming E and H launches, none
+// of which the pass reads) and the hydrodynamic currents (they read E^n, the
+// currents and densities).
+template <typename T, bool RING, bool TFSF, bool HYDRO>
+__global__ void __launch_bounds__(kFlatThreads, 2)
+    h_flat(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
+           const __grid_constant__ LineArgs line, size_t probe_id, const __grid_constant__ FlatGrid g) {
+  unsigned b = blockIdx.x;
+  if (g.line) {
+    if (b == 0) {
+      line_step_body(line, s, probe_id, line.clk->th);
+      return;
+    }
+    b--;
+  }
+  if (HYDRO) {
+    if (b < g.nrole) {
+      hydro_p_any(s, m, s.clk->th, (int)(b * kFlatThreads + threadIdx.x));
+      return;
+    }
+    b -= g.nrole;
+  }
+  const unsigned kb = b / g.nbx, xb = b - kb * g.nbx;
+  h_flat_cells<T, RING, TFSF>(s, xb * kFlatThreads + threadIdx.x, (int)kb * g.kz, g.kz);
 }
 
 // E pass (UPDATE_ex/ey/ez, main.cu:1048-1912) of the vector vq, planes k0 ..
@@ -307,7 +376,7 @@ __global__ void __launch_bounds__(kFlatThreads, 2) h_flat(const __grid_constant_
 // order z, y, x).  The E half of CORRECT_X/Y/Z goes in before the update.
 // Dispersive components are left to the dispersive-cell kernels, which run
 // beside this one: a vector with such a cell stores lane by lane.
-template <typename T, int U>
+template <typename T, bool RING, bool TFSF>
 __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, int k0, int kz) {
   constexpr int N = Vec<T>::N;
   const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
@@ -331,45 +400,62 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
   const bool inbox = i0 + N > s.mat_lo[0] && i0 < s.mat_hi[0] && j >= s.mat_lo[1] && j < s.mat_hi[1];
   const int xs = s.cp[0].Nc <= 0 ? -1 : i0 < s.cp[0].Wn ? i0 : (i0 + N > s.cp[0].fb ? i0 - s.cp[0].fb + s.cp[0].Wn : -1);
   const bool yfar = j >= s.cp[1].F;
-  const int ys = s.cp[1].Nc <= 0 ? -1 : j <= s.cp[1].Nc ? j : (yfar ? j - s.cp[1].F : -1);
+  const int ys = s.cp[1].Nc <= 0 ? -1 : j <= s.cp[1].Nc ? j : (yfar ? j - s.cp[1].F + NZ * (s.cp[1].Nc + 1) : -1);
   const int Ncz = s.cp[2].Nc, Fz = s.cp[2].F;
   const bool edge = lane == 0 || i0 == 0;
   const int ox = i0 > 0 ? -1 : (per ? PX - 1 : 0);
-  const bool tfsf = s.incE != nullptr;
+  const unsigned face = TFSF && s.incE ? flat_faces(s, 1, i0, j) : 0u;
   T check = T(0);
   const unsigned bm = (unsigned)max(k0 - 1, 0) * plane + c0;
   Vec<T> hxm = ldgv(s.H[0] + bm), hym = ldgv(s.H[1] + bm);
   const int k1 = min(k0 + kz, NZ);
-#pragma unroll U
+  FlatRing<T> ring;
+  int st = 0;
+  auto issue = [&](int stage, int k) {
+    if (k < k1) {
+      const unsigned b = (unsigned)k * plane + c0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        ring.issue(stage, c, s.H[c] + b);
+        ring.issue(stage, 3 + c, s.E[c] + b);
+      }
+    }
+    ring.commit();
+  };
+  if (RING) {
+    ring.init();
+#pragma unroll
+    for (int q = 0; q < kFlatRing - 1; q++) issue(q, k0 + q);
+  }
+#pragma unroll 1
   for (int k = k0; k < k1; k++) {
     const unsigned b = (unsigned)k * plane + c0;
     const bool okz = k < NZ - 1, hasz = k > 0;
     // every load of the plane
-    const Vec<T> hx = ldgv(s.H[0] + b), hy = ldgv(s.H[1] + b), hz = ldgv(s.H[2] + b);
     const Vec<T> hxj = ldgv(s.H[0] + b + oj), hzj = ldgv(s.H[2] + b + oj);
-    Vec<T> ex = ldv(s.E[0] + b), ey = ldv(s.E[1] + b), ez = ldv(s.E[2] + b);
+    Vec<T> hx, hy, hz, ex, ey, ez;
+    if (!RING) {
+      hx = ldgv(s.H[0] + b); hy = ldgv(s.H[1] + b); hz = ldgv(s.H[2] + b);
+      ex = ldv(s.E[0] + b); ey = ldv(s.E[1] + b); ez = ldv(s.E[2] + b);
+    }
     T hyi = T(0), hzi = T(0);
     if (edge) { hyi = ldg(s.H[1] + b + ox); hzi = ldg(s.H[2] + b + ox); }
     const T ikz = ldg(s.cp[2].inv_ked + k);
-    T *px0 = nullptr, *px1 = nullptr, *py0 = nullptr, *py1 = nullptr, *pz0 = nullptr, *pz1 = nullptr;
+    unsigned ozo = 0, oxo = 0, oyo = 0;  // offsets in the psi arrays
     Vec<T> ox0, ox1, oy0, oy1, oz0, oz1;
     int zs = -1;
     if (okz && Ncz > 0) zs = k <= Ncz ? k : (k >= Fz ? k - Fz + Ncz + 1 : -1);
     if (zs >= 0) {
-      const unsigned o = (unsigned)zs * plane + c0;
-      pz0 = s.psiE_N[0][1] + o; pz1 = s.psiE_N[1][0] + o;
-      oz0 = ldv(pz0); oz1 = ldv(pz1);
+      ozo = (unsigned)zs * plane + c0;
+      oz0 = ldv(s.psiE_N[0][1] + ozo); oz1 = ldv(s.psiE_N[1][0] + ozo);
     }
     if (ys >= 0 && okz) {
-      const unsigned o = ((unsigned)k * (s.cp[1].Nc + 1) + ys) * PX + i0;
-      py0 = (yfar ? s.psiE_F[0][0] : s.psiE_N[0][0]) + o;
-      py1 = (yfar ? s.psiE_F[2][1] : s.psiE_N[2][1]) + o;
-      oy0 = ldv(py0); oy1 = ldv(py1);
+      oyo = ((unsigned)k * (s.cp[1].Nc + 1) + ys) * PX + i0;
+      oy0 = ldv(s.psiE_N[0][0] + oyo); oy1 = ldv(s.psiE_N[2][1] + oyo);
     }
     if (xs >= 0 && okz) {
-      const unsigned o = ((unsigned)k * NY + j) * s.cp[0].W + xs;
-      px0 = s.psiE_N[1][1] + o; px1 = s.psiE_N[2][0] + o;
-      ox0 = ldv(px0); ox1 = ldv(px1);
+      oxo = ((unsigned)k * NY + j) * s.cp[0].W + xs;
+      ox0 = ldv(s.psiE_N[1][1] + oxo); ox1 = ldv(s.psiE_N[2][0] + oxo);
     }
     // dielectric classes and dispersive components
     Vec<T> ceh;
@@ -387,13 +473,46 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
         if (m >> 3) ceh.v[l] = s.ceh[m >> 3];
       }
     }
+    if (RING) {
+      if (k + 1 < k1) {  // the next plane's psi
+        if (xs >= 0) {
+          const unsigned o = ((unsigned)(k + 1) * NY + j) * s.cp[0].W + xs;
+          flat_touch(s.psiE_N[1][1] + o);
+          flat_touch(s.psiE_N[2][0] + o);
+        }
+        if (ys >= 0) {
+          const unsigned o = ((unsigned)(k + 1) * (s.cp[1].Nc + 1) + ys) * PX + i0;
+          flat_touch(s.psiE_N[0][0] + o);
+          flat_touch(s.psiE_N[2][1] + o);
+        }
+      }
+      ring.wait();
+      issue(st == 0 ? kFlatRing - 1 : st - 1, k + (kFlatRing - 1));
+      hx = ring.get(st, 0, T(0)); hy = ring.get(st, 1, T(0)); hz = ring.get(st, 2, T(0));
+      ex = ring.get(st, 3, T(0)); ey = ring.get(st, 4, T(0)); ez = ring.get(st, 5, T(0));
+      st = st == kFlatRing - 1 ? 0 : st + 1;
+    }
+    T fx = T(0), fy = T(0);  // TFSF increments
+    if (TFSF && face && k >= s.tf.Tz && k < NZ - s.tf.Tz) {
+      if (face & 15u) fx = s.incE[tfsf_inc_at(0, (face >> 8) & 1, 1, NZ) + k];
+      if (face & 240u) fy = s.incE[tfsf_inc_at(1, (face >> 9) & 1, 0, NZ) + k];
+    }
     {
       const T a = __shfl_up_sync(0xFFFFFFFFu, hy.v[N - 1], 1), c = __shfl_up_sync(0xFFFFFFFFu, hz.v[N - 1], 1);
       if (!edge) { hyi = a; hzi = c; }
     }
     const unsigned wx = hasz && okz ? cx & ~mx : 0u, wy = hasz && okz ? cy & ~my : 0u, wz = okz ? cz & ~mz : 0u;
     const bool whole = (mx | my | mz) == 0;
-    if (tfsf && k >= s.tf.Tz && k <= NZ - s.tf.Tz) e_flat_tfsf(s, i0, j, k, ex, ey, ez);
+    // the E half of CORRECT_X/Y/Z, before the update
+    if (TFSF && face) {
+      add_lanes(ez, face & 15u, fx);
+      add_lanes(ez, (face >> 4) & 15u, fy);
+    }
+    if (TFSF && s.incE && (k == s.tf.Tz || k == NZ - s.tf.Tz)) {
+      const int side = k == NZ - s.tf.Tz, Tx = s.tf.Tx, Ty = s.tf.Ty;
+      if (j >= Ty && j <= NY - Ty) add_lanes(ex, lanes_in<N>(i0, Tx, NX - Tx), s.incE[tfsf_inc_at(2, side, 0, NZ) + k]);
+      if (j >= Ty && j < NY - Ty) add_lanes(ey, lanes_in<N>(i0, Tx, min(NX, NX - Tx + 1)), s.incE[tfsf_inc_at(2, side, 1, NZ) + k]);
+    }
     Vec<T> dyz, dzy, dzx, dxz, dxy, dyx;  // d(hz)/dy, d(hy)/dz, d(hx)/dz, d(hz)/dx, d(hy)/dx, d(hx)/dy
 #pragma unroll
     for (int l = 0; l < N; l++) {
@@ -414,25 +533,26 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
     // CPML (cells with i < NX-1, j < NY-1, k < NZ-1: the masks hold these)
     if (zs >= 0) {
       const T bz = ldg(s.cp[2].be + k), cc = ldg(s.cp[2].ce + k);
-      if (wx) psi_vec(pz0, oz0, &bz, &cc, false, s.cp[2].inv_d, dzy, vx, T(-1), ceh, wx, whole);
-      if (wy) psi_vec(pz1, oz1, &bz, &cc, false, s.cp[2].inv_d, dzx, vy, T(1), ceh, wy, whole);
+      if (wx) psi_vec(s.psiE_N[0][1] + ozo, oz0, &bz, &cc, false, s.cp[2].inv_d, dzy, vx, T(-1), ceh, wx, whole);
+      if (wy) psi_vec(s.psiE_N[1][0] + ozo, oz1, &bz, &cc, false, s.cp[2].inv_d, dzx, vy, T(1), ceh, wy, whole);
     }
     if (ys >= 0 && okz) {
       const T by = ldg(s.cp[1].be + j), cc = ldg(s.cp[1].ce + j);
-      if (wx) psi_vec(py0, oy0, &by, &cc, false, s.cp[1].inv_d, dyz, vx, T(1), ceh, wx, whole);
-      if (wz) psi_vec(py1, oy1, &by, &cc, false, s.cp[1].inv_d, dyx, vz, T(-1), ceh, wz, whole);
+      if (wx) psi_vec(s.psiE_N[0][0] + oyo, oy0, &by, &cc, false, s.cp[1].inv_d, dyz, vx, T(1), ceh, wx, whole);
+      if (wz) psi_vec(s.psiE_N[2][1] + oyo, oy1, &by, &cc, false, s.cp[1].inv_d, dyx, vz, T(-1), ceh, wz, whole);
     }
     if (xs >= 0 && okz) {
       const Vec<T> bx = ldgv(s.cp[0].be + i0), cc = ldgv(s.cp[0].ce + i0), cy_ = ldgv(s.cp[0].ce_ey + i0);
-      if (wy) psi_vec(px0, ox0, bx.v, cy_.v, true, s.cp[0].inv_d, dxz, vy, T(-1), ceh, wy, whole);
-      if (wz) psi_vec(px1, ox1, bx.v, cc.v, true, s.cp[0].inv_d, dxy, vz, T(1), ceh, wz, whole);
+      if (wy) psi_vec(s.psiE_N[1][1] + oxo, ox0, bx.v, cy_.v, true, s.cp[0].inv_d, dxz, vy, T(-1), ceh, wy, whole);
+      if (wz) psi_vec(s.psiE_N[2][0] + oxo, ox1, bx.v, cc.v, true, s.cp[0].inv_d, dxy, vz, T(1), ceh, wz, whole);
     }
     if (whole) {
 #pragma unroll
       for (int l = 0; l < N; l++) {
-        if ((wx >> l) & 1) { ex.v[l] = vx.v[l]; check += vx.v[l]; }
-        if ((wy >> l) & 1) { ey.v[l] = vy.v[l]; check += vy.v[l]; }
-        if ((wz >> l) & 1) { ez.v[l] = vz.v[l]; check += vz.v[l]; }
+        if ((wx >> l) & 1) ex.v[l] = vx.v[l];
+        if ((wy >> l) & 1) ey.v[l] = vy.v[l];
+        if ((wz >> l) & 1) ez.v[l] = vz.v[l];
+        check += ex.v[l] + ey.v[l] + ez.v[l];
       }
       if (wx) stv(s.E[0] + b, ex);
       if (wy) stv(s.E[1] + b, ey);
@@ -452,12 +572,25 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
   if (!isfinite(check)) atomicOr(s.nonfinite, 1);
 }
 
-template <typename T, int U>
-__global__ void __launch_bounds__(kFlatThreads, 2) e_flat(const __grid_constant__ SimView<T> s, unsigned nbx, int kz) {
-  pdl_launch_dependents();
-  const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
-  e_flat_cells<T, U>(s, xb * kFlatThreads + threadIdx.x, (int)kb * kz, kz);
-  pdl_wait();
+// The E launch of a step: the E pass and the dispersive cells (KIND 1 = the
+// local model, 2 = the hydrodynamic model), which write disjoint cells.
+template <typename T, bool RING, bool TFSF, int KIND>
+__global__ void __launch_bounds__(kFlatThreads, 2)
+    e_flat(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
+           const __grid_constant__ FlatGrid g) {
+  unsigned b = blockIdx.x;
+  if (b == 0 && threadIdx.x == 0) s.clk->th = s.clk->t;
+  if (KIND) {
+    if (b < g.nrole) {
+      const int q = (int)(b * kFlatThreads + threadIdx.x), t = s.clk->t - 1;
+      if (KIND == 1) metal_e_cell(s, m, t, q);
+      else hydro_e_any(s, m, t, q);
+      return;
+    }
+    b -= g.nrole;
+  }
+  const unsigned kb = b / g.nbx, xb = b - kb * g.nbx;
+  e_flat_cells<T, RING, TFSF>(s, xb * kFlatThreads + threadIdx.x, (int)kb * g.kz, g.kz);
 }
 
 }  // namespace fdtd

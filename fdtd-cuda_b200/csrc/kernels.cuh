@@ -45,6 +45,15 @@ __device__ __forceinline__ size_t fidx(int PX, size_t plane, int i, int j, int k
   return (size_t)k * plane + (size_t)j * PX + i;
 }
 
+// Programmatic dependent launch.  A kernel that triggers lets the launch
+// after it on its stream, when that launch carries a programmatic
+// dependency, start its CTAs as soon as all of this one's have started;
+// griddepcontrol.wait in the later kernel then waits for the earlier one to
+// finish (and its writes to be visible).  Both are no-ops in a launch
+// without a programmatic dependency.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // ---------------------------------------------------------------------
 // TFSF helpers (CORRECT_X/Y/Z, main.cu:369-758)
 
@@ -272,6 +281,8 @@ struct LineArgs {
   double* probe;        // [t][3]
   int probe_cap;
   int dft_every;        // 0 = no DFT sampling
+  const TfsfInc* inc;   // TFSF increments to tabulate from the updated line (0 = none)
+  int ninc, nz;
 };
 
 // E buffer of the line current at step parity `par` (the other one receives
@@ -287,58 +298,103 @@ __device__ __forceinline__ const double* line_e_before(const LineArgs& a, int af
   return line_e(a, a.clk->t - after_line);
 }
 
+// coef * (incident value) / d with the sign, as tfsf_term adds it (boundary.cuh)
 template <typename T>
-__device__ __forceinline__ void line_step_body(const LineArgs& a, const SimView<T>& s, size_t probe_id) {
-  const int t = a.clk->t;
-  const double* ec = line_e(a, t);
+__device__ __forceinline__ void tfsf_increment(const LineArgs& a, const SimView<T>& s, const TfsfInc& x, const double* e,
+                                               T* incH) {
+  const int ax = (x.meta >> 1) & 3, f = (x.meta >> 3) & 3;
+  const bool eh = (x.meta >> 5) & 1;
+  const double* line = eh ? a.h_inc : e;
+  const T v = (T)(((1 - x.dp) * line[x.idx] + x.dp * line[x.idx + 1]) * (double)(eh ? s.tf.fh[f] : s.tf.fe[f]));
+  const T w = (eh ? s.ceh[x.meta >> 6] : s.che) * v / s.dxyz[ax];
+  (eh ? s.incE : incH)[x.dst] = (x.meta & 1) ? w : -w;
+}
+
+// Step t of the line, by one block.  Loads go out four rounds at a time: one
+// block hides no latency by itself.
+template <typename T>
+__device__ __forceinline__ void line_step_body(const LineArgs& a, const SimView<T>& s, size_t probe_id, int t) {
+  constexpr int R = 4;
+  const double* __restrict__ ec = line_e(a, t);
   double* e = line_e(a, t + 1);
+  const int n = blockDim.x;
+  const double m1 = a.clk->e1, m2 = a.clk->e2;
   // probe: E after step t-1 (OUT.txt records it at the top of step t)
   if (threadIdx.x < 3 && t >= 1 && t - 1 < a.probe_cap)
     a.probe[3 * (size_t)(t - 1) + threadIdx.x] = (double)s.E[threadIdx.x][probe_id];
-  for (int q = threadIdx.x; q < a.L - 1; q += blockDim.x)
-    a.h_inc[q] = a.h_inc[q] - a.ch * (ec[q + 1] - ec[q]);
+  for (int q0 = threadIdx.x; q0 < a.L - 1; q0 += R * n) {
+    double h[R], l[R], r[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      const int q = q0 + u * n;
+      if (q < a.L - 1) { h[u] = a.h_inc[q]; l[u] = ec[q]; r[u] = ec[q + 1]; }
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      const int q = q0 + u * n;
+      if (q < a.L - 1) a.h_inc[q] = h[u] - a.ch * (r[u] - l[u]);
+    }
+  }
   __syncthreads();
-  for (int q = threadIdx.x + 1; q < a.L - 1; q += blockDim.x)
-    e[q] = ec[q] - a.ce * (a.h_inc[q] - a.h_inc[q - 1]);
-  __syncthreads();
+  for (int q0 = threadIdx.x + 1; q0 < a.L - 1; q0 += R * n) {
+    double h[R], l[R], c[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      const int q = q0 + u * n;
+      if (q < a.L - 1) { h[u] = a.h_inc[q]; l[u] = a.h_inc[q - 1]; c[u] = ec[q]; }
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      const int q = q0 + u * n;
+      if (q < a.L - 1) {
+        double v = c[u] - a.ce * (h[u] - l[u]);
+        if (q == 1) {  // Mur ends: the neighbour's new value is in hand
+          e[0] = m1 + a.mur * (v - ec[0]);
+          a.clk->e1 = v;
+        }
+        if (q == a.L - 2) {
+          double w = m2 + a.mur * (v - ec[a.L - 1]);
+          a.clk->e2 = v;
+          if (a.src == a.L - 1 && t < a.tmax) w += a.pulse[t];
+          e[a.L - 1] = w;
+        }
+        if (q == a.src && t < a.tmax) v += a.pulse[t];
+        e[q] = v;
+      }
+    }
+  }
   if (threadIdx.x == 0) {
-    e[0] = a.clk->e1 + a.mur * (e[1] - ec[0]);
-    e[a.L - 1] = a.clk->e2 + a.mur * (e[a.L - 2] - ec[a.L - 1]);
-    a.clk->e1 = e[1];
-    a.clk->e2 = e[a.L - 2];
-    if (t < a.tmax) e[a.src] += a.pulse[t];
     // reserve this step's slot in the DFT sample ring (ScattAbs runs when
     // t % 4 == 0, main.cu:2920)
     if (a.dft_every > 0 && t % a.dft_every == 0) {
-      const int n = a.clk->nsamp;
-      if (n < kRingSlots) {
-        const int slot = a.clk->base + n;
+      const int ns = a.clk->nsamp;
+      if (ns < kRingSlots) {
+        const int slot = a.clk->base + ns;
         a.clk->samp_slot = slot;
         a.clk->samp_t[slot] = t;
-        a.clk->nsamp = n + 1;
+        a.clk->nsamp = ns + 1;
       } else {
         a.clk->samp_slot = -1;  // half full: the caller skipped a contraction
       }
     }
     a.clk->t = t + 1;
   }
+  if (a.ninc > 0) {
+    __syncthreads();
+    T* incH = s.incH + (size_t)((t + 1) & 1) * 12 * a.nz;
+    for (int q = threadIdx.x; q < a.ninc; q += n) tfsf_increment(a, s, a.inc[q], e, incH);
+  }
 }
-// Programmatic dependent launch.  A kernel that triggers lets the launch
-// after it on its stream, when that launch carries a programmatic
-// dependency, start its CTAs as soon as all of this one's have started;
-// griddepcontrol.wait in the later kernel then waits for the earlier one to
-// finish (and its writes to be visible).  Both are no-ops in a launch
-// without a programmatic dependency.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 // The line step triggers at once: the H pass launched after it reads
 // nothing it writes (and waits for it at its own end).
 template <typename T>
 __global__ void __launch_bounds__(1024) line_step(const __grid_constant__ LineArgs a, const __grid_constant__ SimView<T> s,
                                                   size_t probe_id) {
   pdl_launch_dependents();
-  line_step_body(a, s, probe_id);
+  const int t = a.clk->t;
+  __syncthreads();  // every thread has read the clock before it moves on
+  line_step_body(a, s, probe_id, t);
+  if (threadIdx.x == 0) a.clk->th = t + 1;
 }
 
 template <typename T>
@@ -398,13 +454,39 @@ __device__ __forceinline__ size_t rec_row(int t, int base, int rows) {
   return (size_t)(d < 0 ? d + rows : d);
 }
 
+// The step's TFSF increments on the faces (CORRECT_X/Y/Z, main.cu:369-758) of
+// a plane wave along z: per face (axis, side) and tangential component (slot
+// 0 = the axis after the normal, 1 = the one after that) one value per z
+// index, the sign included.  E_z and H_z of the wave are zero, so on the x and
+// y faces only the z component takes one.  The line step fills them.
+__host__ __device__ __forceinline__ int tfsf_inc_at(int axis, int side, int slot, int NZ) {
+  return ((axis * 2 + side) * 2 + slot) * NZ;
+}
+// E of component c of one cell with its E-half corrections, in the order X, Y,
+// Z (tfsf_e_walk's ranges).
+template <typename T>
+__device__ __forceinline__ T tfsf_e_cell(const SimView<T>& s, int c, int i, int j, int k, T v) {
+  const int p[3] = {i, j, k}, N3[3] = {s.NX, s.NY, s.NZ}, t3[3] = {s.tf.Tx, s.tf.Ty, s.tf.Tz};
+#pragma unroll
+  for (int ax = 0; ax < 3; ax++) {
+    if (ax == c) continue;
+    bool in = true;
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+      if (b != ax) in = in && p[b] >= t3[b] && (b == c ? p[b] < N3[b] - t3[b] : p[b] <= N3[b] - t3[b]);
+    if (!in) continue;
+    const T* inc = s.incE + tfsf_inc_at(ax, 0, (c - ax + 3) % 3 - 1, s.NZ) + k;
+    if (p[ax] == t3[ax]) v += inc[0];
+    else if (p[ax] == N3[ax] - t3[ax]) v += inc[2 * s.NZ];
+  }
+  return v;
+}
+
 // Non-hydrodynamic dispersive update of all three components (they do not
 // couple within a step).  pd ring: n = t%3, n-1 = (t+2)%3, new = (t+1)%3.
 template <typename T>
-__device__ __forceinline__ void metal_e_body(const SimView<T>& s, const MetalView<T>& m, const DevClock* clk) {
-  const int t = clk->t - 1;
+__device__ __forceinline__ void metal_e_cell(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
   const int rn = t % 3, rn1 = (t + 2) % 3, rnew = (t + 1) % 3;
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
   int c = 0;
   while (c < 3 && q >= m.n[c]) { q -= m.n[c]; c++; }
   if (c >= 3) return;
@@ -413,8 +495,9 @@ __device__ __forceinline__ void metal_e_body(const SimView<T>& s, const MetalVie
   const size_t id = fidx(s.PX, s.plane, i, j, k);
   const unsigned mb = s.mat[id];
   const T ceh = s.ceh[mb >> 3];
-  // the E half of CORRECT_* has already been added by tfsf_e_apply
-  const T v = s.E[c][id];
+  // the E half of CORRECT_*: added by tfsf_apply, or here from the increments
+  T v = s.E[c][id];
+  if (s.incE) v = tfsf_e_cell(s, c, i, j, k, v);
   T da, db;
   const T curl = curl_h_at(s, c, i, j, k, &da, &db);
   const double pdn = m.pd[c][rn][sl], pdn1 = m.pd[c][rn1][sl];
@@ -467,7 +550,7 @@ __device__ __forceinline__ void metal_e_body(const SimView<T>& s, const MetalVie
 template <typename T>
 __global__ void metal_e(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m, const DevClock* clk) {
   pdl_launch_dependents();  // the E pass after it touches none of its cells
-  metal_e_body(s, m, clk);
+  metal_e_cell(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
 }
 
 // Neighbour values of a dispersive cell for the hydrodynamic model.  nbr
@@ -482,12 +565,11 @@ __device__ __forceinline__ void hydro_neighbours(const MetalView<T>& m, int q, i
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     const int rp = (a < cphase) ? (t + 1) % 3 : t % 3;
-    const int rn = ((a < cphase) ? t + 1 : t) & 1;
 #pragma unroll
     for (int x = 0; x < 4; x++) {
       const int sl = nb[a * 4 + x];
       P[a][x] = sl >= 0 ? m.pd[a][rp][sl] : 0.0;
-      N[a][x] = sl >= 0 ? m.nd[a][rn][sl] : 0.0;
+      N[a][x] = sl >= 0 ? m.nd[a][rp][sl] : 0.0;
     }
   }
 }
@@ -526,15 +608,11 @@ __device__ __forceinline__ double hydro_current(const MetalView<T>& m, int t, in
          m.dNL * ((gd + gd2 / m.N_EQ) / cb);
 }
 
-// Hydrodynamic E update of one cell of component c (UPDATE_e* hydro
-// branch, main.cu:1220-1271 and mirrors): continuity for the density
-// perturbation, then E with the current source e0 (N_EQ + N) J.
+// The new density N^{n+1} of one cell of component c: the continuity update of
+// UPDATE_e*'s hydro branch (main.cu:1220-1271 and mirrors).
 template <typename T, int c>
-__device__ __forceinline__ void hydro_e_cell(const SimView<T>& s, const MetalView<T>& m, int t, int4 e,
-                                             const double P[3][4], const double N[3][4], double jd) {
-  const int i = e.x, j = e.y, k = e.z, sl = e.w;
-  const size_t id = fidx(s.PX, s.plane, i, j, k);
-  const T ceh = s.ceh[s.mat[id] >> 3];
+__device__ __forceinline__ double hydro_density(const MetalView<T>& m, int t, int sl, const double P[3][4],
+                                                const double N[3][4]) {
   double V1[3], V2[3], N1[3], N2[3];
 #pragma unroll
   for (int a = 0; a < 3; a++) {
@@ -547,7 +625,7 @@ __device__ __forceinline__ void hydro_e_cell(const SimView<T>& s, const MetalVie
       N2[a] = 0.5 * (N[a][2] + N[a][3]);
     }
   }
-  const double ndm1 = m.nd[c][(t + 1) & 1][sl];  // N^{n-1}
+  const double ndm1 = m.nd[c][(t + 2) % 3][sl];  // N^{n-1}
   const double k2 = 2.0 * m.dt * m.inv_dx;
   // an adjoint design cell scales its current and density updates and
   // blends its coupling coefficients by rho (rho = 0: a vacuum cell with
@@ -567,7 +645,19 @@ __device__ __forceinline__ void hydro_e_cell(const SimView<T>& s, const MetalVie
     nd = ndm1 - k2 * ((N1[0] * V1[0] - N2[0] * V2[0]) + (N1[1] * V1[1] - N2[1] * V2[1]) +
                       0.5 * (V1[2] - V2[2]) +
                       ((V1[0] - V2[0]) + (V1[1] - V2[1]) + 0.5 * (V1[2] - V2[2])) * m.N_EQ);
-  if (blend) nd = r * nd;
+  return blend ? r * nd : nd;
+}
+
+// Hydrodynamic E update of one cell of component c from its new density and
+// current: the current source e0 (N_EQ + N) J.
+template <typename T, int c>
+__device__ __forceinline__ void hydro_e_cell(const SimView<T>& s, const MetalView<T>& m, int t, int4 e, double nd,
+                                             double jd) {
+  const int i = e.x, j = e.y, k = e.z, sl = e.w;
+  const size_t id = fidx(s.PX, s.plane, i, j, k);
+  const T ceh = s.ceh[s.mat[id] >> 3];
+  const bool blend = m.rho[c] != nullptr;
+  const double r = blend ? (double)m.rho[c][sl] : 1.0;
   const T v = s.E[c][id];
   T da, db;
   const T curl = curl_h_at(s, c, i, j, k, &da, &db);
@@ -607,12 +697,13 @@ __device__ __forceinline__ void hydro_e_cell(const SimView<T>& s, const MetalVie
   m.cpn1[c][1][sl] = cpn1;
   m.cpn[c][0][sl] = ncp0;
   m.cpn[c][1][sl] = ncp1;
-  m.nd[c][(t + 1) & 1][sl] = nd;  // becomes "prev" after the parity flip
   nv = cpml_e_all(s, c, i, j, k, da, db, nv, ceh);
   if (!isfinite((double)nv)) atomicOr(s.nonfinite, 1);
   s.E[c][id] = nv;
 }
 
+// Currents of one cell (UpdateHydroP*), and for an x cell the new density,
+// which needs the state from before this step only.
 template <typename T, int c>
 __device__ __forceinline__ void hydro_p_cell(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
   const int4 e = m.cell[c][q];
@@ -620,7 +711,7 @@ __device__ __forceinline__ void hydro_p_cell(const SimView<T>& s, const MetalVie
   hydro_neighbours<T, c, 0>(m, q, t, P, N);
   const size_t id = fidx(s.PX, s.plane, e.x, e.y, e.z);
   double jd = hydro_current<T, c>(m, t, e.w, P, N, s.E[c][id], m.en[c][e.w]);
-  if (m.rho[c]) jd *= (double)m.rho[c][e.w];  // adjoint design cell (see hydro_e_cell)
+  if (m.rho[c]) jd *= (double)m.rho[c][e.w];  // adjoint design cell (see hydro_density)
   if (m.hrec) {
     // J^{n-1}, J^n, J^{n+1}, N^{n-1}, N^n of the slot; N^{n+1} follows in
     // hydro_e_cell
@@ -629,43 +720,79 @@ __device__ __forceinline__ void hydro_p_cell(const SimView<T>& s, const MetalVie
     h[0] = (T)m.pd[c][(t + 2) % 3][e.w];
     h[S] = (T)m.pd[c][t % 3][e.w];
     h[2 * S] = (T)jd;
-    h[3 * S] = (T)m.nd[c][(t + 1) & 1][e.w];
-    h[4 * S] = (T)m.nd[c][t & 1][e.w];
+    h[3 * S] = (T)m.nd[c][(t + 2) % 3][e.w];
+    h[4 * S] = (T)m.nd[c][t % 3][e.w];
   }
   m.pd[c][(t + 1) % 3][e.w] = jd;
-  if (c == 0) hydro_e_cell<T, 0>(s, m, t, e, P, N, jd);
+  if (c == 0) m.nd[0][(t + 1) % 3][e.w] = hydro_density<T, 0>(m, t, e.w, P, N);
 }
-
-// Phase 1 of the hydrodynamic step: UpdateHydroP* for every dispersive
-// cell, and the Ex update for the x cells (which needs only its own new
-// current and the state from before this step).
+// Cell q of the three components' lists taken after one another.
 template <typename T>
-__global__ void hydro_p_ex(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
-                           const DevClock* clk) {
-  pdl_launch_dependents();  // the next phase waits for this one itself; the E pass touches none of its cells
-  const int t = clk->t - 1;
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void hydro_p_any(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
+  int c = 0;
+  while (c < 3 && q >= m.n[c]) { q -= m.n[c]; c++; }
+  if (c == 0) hydro_p_cell<T, 0>(s, m, t, q);
+  else if (c == 1) hydro_p_cell<T, 1>(s, m, t, q);
+  else if (c == 2) hydro_p_cell<T, 2>(s, m, t, q);
+}
+// E of one cell once every new current and every new x density are there: an
+// x cell reads its density, a y cell computes its own from neighbours that are
+// all new, a z cell needs the new y densities of up to four neighbours and
+// computes them again (the y cells store theirs at the same time), so that the
+// three components run side by side.
+template <typename T>
+__device__ __forceinline__ void hydro_e_any(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
   int c = 0;
   while (c < 3 && q >= m.n[c]) { q -= m.n[c]; c++; }
   if (c >= 3) return;
-  if (c == 0) hydro_p_cell<T, 0>(s, m, t, q);
-  else if (c == 1) hydro_p_cell<T, 1>(s, m, t, q);
-  else hydro_p_cell<T, 2>(s, m, t, q);
+  const int rnew = (t + 1) % 3;
+  if (c == 0) {
+    const int4 e = m.cell[0][q];
+    hydro_e_cell<T, 0>(s, m, t, e, m.nd[0][rnew][e.w], m.pd[0][rnew][e.w]);
+  } else if (c == 1) {
+    const int4 e = m.cell[1][q];
+    double P[3][4], N[3][4];
+    hydro_neighbours<T, 1, 1>(m, q, t, P, N);
+    const double nd = hydro_density<T, 1>(m, t, e.w, P, N);
+    m.nd[1][rnew][e.w] = nd;
+    hydro_e_cell<T, 1>(s, m, t, e, nd, m.pd[1][rnew][e.w]);
+  } else {
+    const int4 e = m.cell[2][q];
+    double N1[4];
+    const int* nb = m.nbr[2] + (size_t)q * 12 + 4;
+#pragma unroll 1
+    for (int x = 0; x < 4; x++) {
+      const int sl = nb[x];
+      N1[x] = 0.0;
+      if (sl >= 0) {
+        double P[3][4], N[3][4];
+        hydro_neighbours<T, 1, 1>(m, sl, t, P, N);  // a cell's list entry is its slot
+        N1[x] = hydro_density<T, 1>(m, t, sl, P, N);
+      }
+    }
+    double P[3][4], N[3][4];
+    hydro_neighbours<T, 2, 2>(m, q, t, P, N);
+#pragma unroll
+    for (int x = 0; x < 4; x++) N[1][x] = N1[x];
+    const double nd = hydro_density<T, 2>(m, t, e.w, P, N);
+    m.nd[2][rnew][e.w] = nd;
+    hydro_e_cell<T, 2>(s, m, t, e, nd, m.pd[2][rnew][e.w]);
+  }
 }
 
-// Phases 2 and 3: the Ey, then the Ez update.
-template <typename T, int c>
+// The hydrodynamic step as two launches of its own: the currents, then E.
+template <typename T>
+__global__ void hydro_p(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
+                        const DevClock* clk) {
+  pdl_launch_dependents();  // the next launch waits for this one itself; the E pass touches none of its cells
+  hydro_p_any(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+}
+template <typename T>
 __global__ void hydro_e(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
                         const DevClock* clk) {
   pdl_launch_dependents();
-  pdl_wait();  // the previous phase has finished
-  const int t = clk->t - 1;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= m.n[c]) return;
-  const int4 e = m.cell[c][q];
-  double P[3][4], N[3][4];
-  hydro_neighbours<T, c, c>(m, q, t, P, N);
-  hydro_e_cell<T, c>(s, m, t, e, P, N, m.pd[c][(t + 1) % 3][e.w]);
+  pdl_wait();  // the currents are there
+  hydro_e_any(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
 }
 
 // ---------------------------------------------------------------------

@@ -53,7 +53,7 @@ __global__ void snap_gather(const __grid_constant__ SimView<T> s, const __grid_c
       for (int c = 0; c < 3; c++) {
         const int sl = ps[c];
         p[c] = sl >= 0 ? m.pd[c][(t + 1) % 3][sl] : 0.0;
-        nd[c] = (sl >= 0 && m.hydro) ? m.nd[c][t & 1][sl] : 0.0;
+        nd[c] = (sl >= 0 && m.hydro) ? m.nd[c][t % 3][sl] : 0.0;
       }
       r[a.off_plane + q] = sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
       r[a.off_plane2 + q] = (nd[0] + nd[1] + nd[2]) / 3.0;

@@ -3,7 +3,9 @@
 Both forms do the same operations in the same order per cell, so fields are
 bit-identical: over row lengths of every remainder of the 16-byte vector and
 of the padded pitch, grids of fewer planes than a thread takes, dispersive
-cells inside the CPML, dielectric classes and periodic x and y.
+cells inside the CPML, dielectric classes and periodic x and y, with the TFSF
+corrections in the passes or in a launch of their own, in the fused step and
+through the split entry points.
 """
 import numpy as np
 import pytest
@@ -13,7 +15,7 @@ from cases import make
 
 pytestmark = pytest.mark.gpu
 
-SPECS = ("flat:1", "flat:5", "flat:8:8", "flat:64:8", "flat:200")
+SPECS = ("flat:1", "flat:5", "flat:2:1", "flat:8:1", "flat:64:1", "flat:200")
 
 
 def fields(name, prec, spec, monkeypatch, steps, **over):
@@ -38,16 +40,49 @@ def agree(name, prec, specs, monkeypatch, steps=150, **over):
         np.testing.assert_array_equal(t, tab)
 
 
+@pytest.mark.parametrize("tfsf", ["0", "1"])
 @pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
 @pytest.mark.parametrize("name", ["sphere_big", "slab", "disks_slab", "hydro", "fixes", "periodic_spheres"])
-def test_direct_passes_agree_with_the_staged_ones(name, prec, monkeypatch):
+def test_direct_passes_agree_with_the_staged_ones(name, prec, tfsf, monkeypatch):
+    monkeypatch.setenv("FDTD_TFSF", tfsf)
     agree(name, prec, SPECS, monkeypatch)
+
+
+@pytest.mark.parametrize("angles", [dict(inc_phi_deg=30.0), dict(inc_phi_deg=90.0, polar_psi_deg=20.0),
+                                    dict(inc_theta_deg=25.0, inc_phi_deg=40.0, polar_psi_deg=10.0)])
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+def test_every_polarisation_and_oblique_incidence(angles, prec, monkeypatch):
+    """Oblique incidence keeps the TFSF launch whatever is asked for."""
+    monkeypatch.setenv("FDTD_TFSF", "1")
+    agree("slab", prec, ("flat:1", "flat:4:1"), monkeypatch, **angles)
+
+
+@pytest.mark.parametrize("tfsf", ["0", "1"])
+@pytest.mark.parametrize("name", ["sphere_big", "slab", "hydro"])
+def test_split_entry_points_agree_with_the_fused_step(name, tfsf, monkeypatch):
+    """Both in one run too: the clocks of the two forms stay together."""
+    monkeypatch.setenv("FDTD_TFSF", tfsf)
+    a, b = (F.Sim(make(F, name, precision=F.FDTD_FP32)) for _ in range(2))
+    a.step(140)
+    b.step(33)
+    for _ in range(70):
+        b.update_h()
+        b.update_line()
+        b.update_e()
+        b.spectral_accumulate()
+    b.step(37)
+    for c in range(6):
+        np.testing.assert_array_equal(a.field(c), b.field(c))
+    np.testing.assert_array_equal(a.probe(), b.probe())
+    np.testing.assert_array_equal(a.spectra(), b.spectra())
+    a.close()
+    b.close()
 
 
 @pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
 @pytest.mark.parametrize("dx", range(8))
 def test_every_row_remainder(dx, prec, monkeypatch):
-    agree("sphere_au", prec, ("flat:1", "flat:7:8"), monkeypatch, steps=90, NCELLX=21 + dx, NCELLY=22 - dx % 3)
+    agree("sphere_au", prec, ("flat:1", "flat:7:1"), monkeypatch, steps=90, NCELLX=21 + dx, NCELLY=22 - dx % 3)
 
 
 def test_tuned_and_untuned_direct_passes_agree(monkeypatch):
@@ -66,7 +101,7 @@ def test_tuned_and_untuned_direct_passes_agree(monkeypatch):
 
 
 def test_unbuilt_direct_variant_is_rejected(monkeypatch):
-    for spec in ("flat:0", "flat:4:3"):
+    for spec in ("flat:0", "flat:4:2"):
         monkeypatch.setenv("FDTD_PASS", spec)
         with pytest.raises(F.FdtdError) as e:
             F.Sim(make(F, "vacuum", precision=F.FDTD_FP32))
