@@ -92,32 +92,45 @@ __device__ __forceinline__ void flat_touch(const T* p) {
   asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
 }
 
-// CPML of one vector and one axis: psi <- b psi + c diff / d per lane, and
-// the field += sg coef psi; w = lanes that are updated (the others keep psi).
+// CPML of one vector and one axis: psi <- b psi + c diff / d per lane, and the
+// field += sg coef psi.  Lanes whose cell is not updated come with c = 0 (their
+// psi is and stays zero); skip = lanes of dispersive cells, whose psi belongs to
+// the dispersive-cell update.
 template <typename T>
 __device__ __forceinline__ T lane_of(const T& x, int) { return x; }
 template <typename T>
 __device__ __forceinline__ T lane_of(const Vec<T>& x, int l) { return x.v[l]; }
-template <typename T, typename C>
-__device__ __forceinline__ void psi_vec(T* p, const Vec<T>& old, const T* b, const T* c, bool per_lane, T inv_d,
-                                        const Vec<T>& diff, Vec<T>& v, T sg, const C& coef, unsigned w,
-                                        bool whole) {
+template <typename T, typename B, typename C>
+__device__ __forceinline__ void psi_vec(T* p, const Vec<T>& old, const B& b, const Vec<T>& c, T inv_d,
+                                        const Vec<T>& diff, Vec<T>& v, T sg, const C& coef, unsigned skip = 0) {
   constexpr int N = Vec<T>::N;
   Vec<T> ps;
 #pragma unroll
   for (int l = 0; l < N; l++) {
-    const T bl = per_lane ? b[l] : b[0], cl = per_lane ? c[l] : c[0];
-    const T x = rfma(bl, old.v[l], rmul(rmul(cl, diff.v[l]), inv_d));
-    const bool on = (w >> l) & 1;
-    ps.v[l] = on ? x : old.v[l];
-    if (on) v.v[l] = rfma(sg * lane_of(coef, l), x, v.v[l]);
+    ps.v[l] = rfma(lane_of(b, l), old.v[l], rmul(rmul(c.v[l], diff.v[l]), inv_d));
+    v.v[l] = rfma(sg * lane_of(coef, l), ps.v[l], v.v[l]);
   }
-  if (whole) stv(p, ps);
+  if (!skip) stv(p, ps);
   else {
 #pragma unroll
     for (int l = 0; l < N; l++)
-      if ((w >> l) & 1) p[l] = ps.v[l];
+      if (!((skip >> l) & 1)) p[l] = ps.v[l];
   }
+}
+template <typename T>
+__device__ __forceinline__ T sum(const Vec<T>& x) {
+  T r = x.v[0];
+#pragma unroll
+  for (int l = 1; l < Vec<T>::N; l++) r += x.v[l];
+  return r;
+}
+// a coefficient on the lanes of m, 0 on the others
+template <typename T, typename C>
+__device__ __forceinline__ Vec<T> keep_lanes(unsigned m, const C& c) {
+  Vec<T> r;
+#pragma unroll
+  for (int l = 0; l < Vec<T>::N; l++) r.v[l] = (m >> l) & 1 ? lane_of(c, l) : T(0);
+  return r;
 }
 
 // Lanes of the vector at i0 whose cell index lies in [lo, hi).
@@ -175,7 +188,7 @@ __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, i
   // hx and hz are not updated)
   const int oj = j + 1 < NY ? PX : (per ? -(NY - 1) * PX : 0);
   const unsigned lane = threadIdx.x & 31;
-  const unsigned wx = lanes_in<N>(i0, 0, per ? NX : NX - 1);  // lanes with a +x neighbour
+  const unsigned on = lanes_in<N>(i0, 0, per ? NX : NX - 1);  // lanes with a +x neighbour
   const Vec<T> ikx = ldgv(s.cp[0].inv_khd + i0);
   const T iky = ldg(s.cp[1].inv_khd + j);
   const T che = s.che, chh = s.chh;
@@ -291,29 +304,29 @@ __device__ __forceinline__ void h_flat_cells(const SimView<T>& s, unsigned vq, i
     }
     // CPML (cells with every index below N-1, main.cu:829); per axis in the
     // order z, x, y
-    const unsigned wp = hasy && in ? wx : 0u;
-    if (wp) {
+    if (hasy && in) {
       if (zs >= 0) {
-        const T bz = ldg(s.cp[2].bh + k), cz = ldg(s.cp[2].ch + k);
-        psi_vec(s.psiH_N[0][1] + ozo, oz0, &bz, &cz, false, s.cp[2].inv_d, dzy, vx, T(1), che, wp, true);
-        psi_vec(s.psiH_N[1][0] + ozo, oz1, &bz, &cz, false, s.cp[2].inv_d, dzx, vy, T(-1), che, wp, true);
+        const T bz = ldg(s.cp[2].bh + k);
+        const Vec<T> cz = keep_lanes<T>(on, ldg(s.cp[2].ch + k));
+        psi_vec(s.psiH_N[0][1] + ozo, oz0, bz, cz, s.cp[2].inv_d, dzy, vx, T(1), che);
+        psi_vec(s.psiH_N[1][0] + ozo, oz1, bz, cz, s.cp[2].inv_d, dzx, vy, T(-1), che);
       }
       if (xs >= 0 && hask) {
-        const Vec<T> bx = ldgv(s.cp[0].bh + i0), cx = ldgv(s.cp[0].ch + i0);
-        psi_vec(s.psiH_N[1][1] + oxo, ox0, bx.v, cx.v, true, s.cp[0].inv_d, dxz, vy, T(1), che, wp, true);
-        psi_vec(s.psiH_N[2][0] + oxo, ox1, bx.v, cx.v, true, s.cp[0].inv_d, dxy, vz, T(-1), che, wp, true);
+        const Vec<T> bx = ldgv(s.cp[0].bh + i0), cx = ldgv(s.cp[0].ch + i0);  // zero at NX-1
+        psi_vec(s.psiH_N[1][1] + oxo, ox0, bx, cx, s.cp[0].inv_d, dxz, vy, T(1), che);
+        psi_vec(s.psiH_N[2][0] + oxo, ox1, bx, cx, s.cp[0].inv_d, dxy, vz, T(-1), che);
       }
       if (ys >= 0 && hask) {
-        const T by = ldg(s.cp[1].bh + j), cy = ldg(s.cp[1].ch + j);
-        psi_vec(s.psiH_N[0][0] + oyo, oy0, &by, &cy, false, s.cp[1].inv_d, dyz, vx, T(-1), che, wp, true);
-        psi_vec(s.psiH_N[2][1] + oyo, oy1, &by, &cy, false, s.cp[1].inv_d, dyx, vz, T(1), che, wp, true);
+        const T by = ldg(s.cp[1].bh + j);
+        const Vec<T> cy = keep_lanes<T>(on, ldg(s.cp[1].ch + j));
+        psi_vec(s.psiH_N[0][0] + oyo, oy0, by, cy, s.cp[1].inv_d, dyz, vx, T(-1), che);
+        psi_vec(s.psiH_N[2][1] + oyo, oy1, by, cy, s.cp[1].inv_d, dyx, vz, T(1), che);
       }
     }
 #pragma unroll
     for (int l = 0; l < N; l++) {
-      const bool on = (wx >> l) & 1;
       hx.v[l] = vx.v[l];
-      if (on) { hy.v[l] = vy.v[l]; hz.v[l] = vz.v[l]; }
+      if ((on >> l) & 1) { hy.v[l] = vy.v[l]; hz.v[l] = vz.v[l]; }
     }
     // the H half of CORRECT_X/Y/Z
     if (TFSF && face) {
@@ -391,9 +404,8 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
   // lanes whose ex, ey, ez are updated in this column (main.cu:1172, 1476,
   // 1767; every column when periodic, main.cu:1072, 1364, 1668)
   const bool jlo = per || j > 0, jhi = per || j < NY - 1;
-  const unsigned wlo = per ? lanes_in<N>(i0, 0, NX) : lanes_in<N>(i0, 1, NX - 1);
-  const unsigned wall = per ? wlo : lanes_in<N>(i0, 0, NX - 1);
-  const unsigned cx = in && jlo && jhi ? wall : 0u, cy = in && jhi ? wlo : 0u, cz = in && jlo && jhi ? wlo : 0u;
+  const unsigned onx = lanes_in<N>(i0, 0, per ? NX : NX - 1), onyz = onx & ~(!per && i0 == 0 ? 1u : 0u);
+  const bool rowy = in && jhi, rowxz = rowy && jlo;
   const Vec<T> ikx = ldgv(s.cp[0].inv_ked + i0);
   const T iky = ldg(s.cp[1].inv_ked + j);
   const T cee0 = s.cee[0], ceh0 = s.ceh[0];
@@ -406,7 +418,7 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
   const int ox = i0 > 0 ? -1 : (per ? PX - 1 : 0);
   const unsigned face = TFSF && s.incE ? flat_faces(s, 1, i0, j) : 0u;
   T check = T(0);
-  const unsigned bm = (unsigned)max(k0 - 1, 0) * plane + c0;
+  const unsigned bm = (unsigned)min(max(k0 - 1, 0), NZ - 1) * plane + c0;  // (a batch block's groups may start past NZ)
   Vec<T> hxm = ldgv(s.H[0] + bm), hym = ldgv(s.H[1] + bm);
   const int k1 = min(k0 + kz, NZ);
   FlatRing<T> ring;
@@ -501,8 +513,7 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
       const T a = __shfl_up_sync(0xFFFFFFFFu, hy.v[N - 1], 1), c = __shfl_up_sync(0xFFFFFFFFu, hz.v[N - 1], 1);
       if (!edge) { hyi = a; hzi = c; }
     }
-    const unsigned wx = hasz && okz ? cx & ~mx : 0u, wy = hasz && okz ? cy & ~my : 0u, wz = okz ? cz & ~mz : 0u;
-    const bool whole = (mx | my | mz) == 0;
+    const bool upx = rowxz && hasz && okz, upy = rowy && hasz && okz, upz = rowxz && okz;
     // the E half of CORRECT_X/Y/Z, before the update
     if (TFSF && face) {
       add_lanes(ez, face & 15u, fx);
@@ -530,39 +541,37 @@ __device__ __forceinline__ void e_flat_cells(const SimView<T>& s, unsigned vq, i
       vy.v[l] = rfma(ceh.v[l], rcurl(dzx.v[l], ikz, dxz.v[l], ikx.v[l]), rmul(cee0, ey.v[l]));
       vz.v[l] = rfma(ceh.v[l], rcurl(dxy.v[l], ikx.v[l], dyx.v[l], iky), rmul(cee0, ez.v[l]));
     }
-    // CPML (cells with i < NX-1, j < NY-1, k < NZ-1: the masks hold these)
+    // CPML (cells with i < NX-1, j < NY-1, k < NZ-1)
     if (zs >= 0) {
-      const T bz = ldg(s.cp[2].be + k), cc = ldg(s.cp[2].ce + k);
-      if (wx) psi_vec(s.psiE_N[0][1] + ozo, oz0, &bz, &cc, false, s.cp[2].inv_d, dzy, vx, T(-1), ceh, wx, whole);
-      if (wy) psi_vec(s.psiE_N[1][0] + ozo, oz1, &bz, &cc, false, s.cp[2].inv_d, dzx, vy, T(1), ceh, wy, whole);
+      const T bz = ldg(s.cp[2].be + k), cz = ldg(s.cp[2].ce + k);
+      if (upx) psi_vec(s.psiE_N[0][1] + ozo, oz0, bz, keep_lanes<T>(onx, cz), s.cp[2].inv_d, dzy, vx, T(-1), ceh, mx);
+      if (upy) psi_vec(s.psiE_N[1][0] + ozo, oz1, bz, keep_lanes<T>(onyz, cz), s.cp[2].inv_d, dzx, vy, T(1), ceh, my);
     }
     if (ys >= 0 && okz) {
-      const T by = ldg(s.cp[1].be + j), cc = ldg(s.cp[1].ce + j);
-      if (wx) psi_vec(s.psiE_N[0][0] + oyo, oy0, &by, &cc, false, s.cp[1].inv_d, dyz, vx, T(1), ceh, wx, whole);
-      if (wz) psi_vec(s.psiE_N[2][1] + oyo, oy1, &by, &cc, false, s.cp[1].inv_d, dyx, vz, T(-1), ceh, wz, whole);
+      const T by = ldg(s.cp[1].be + j), cy = ldg(s.cp[1].ce + j);
+      if (upx) psi_vec(s.psiE_N[0][0] + oyo, oy0, by, keep_lanes<T>(onx, cy), s.cp[1].inv_d, dyz, vx, T(1), ceh, mx);
+      if (upz) psi_vec(s.psiE_N[2][1] + oyo, oy1, by, keep_lanes<T>(onyz, cy), s.cp[1].inv_d, dyx, vz, T(-1), ceh, mz);
     }
     if (xs >= 0 && okz) {
-      const Vec<T> bx = ldgv(s.cp[0].be + i0), cc = ldgv(s.cp[0].ce + i0), cy_ = ldgv(s.cp[0].ce_ey + i0);
-      if (wy) psi_vec(s.psiE_N[1][1] + oxo, ox0, bx.v, cy_.v, true, s.cp[0].inv_d, dxz, vy, T(-1), ceh, wy, whole);
-      if (wz) psi_vec(s.psiE_N[2][0] + oxo, ox1, bx.v, cc.v, true, s.cp[0].inv_d, dxy, vz, T(1), ceh, wz, whole);
+      const Vec<T> bx = ldgv(s.cp[0].be + i0);
+      if (upy) psi_vec(s.psiE_N[1][1] + oxo, ox0, bx, keep_lanes<T>(onyz, ldgv(s.cp[0].ce_ey + i0)), s.cp[0].inv_d, dxz, vy, T(-1), ceh, my);
+      if (upz) psi_vec(s.psiE_N[2][0] + oxo, ox1, bx, keep_lanes<T>(onyz, ldgv(s.cp[0].ce + i0)), s.cp[0].inv_d, dxy, vz, T(1), ceh, mz);
     }
-    if (whole) {
 #pragma unroll
-      for (int l = 0; l < N; l++) {
-        if ((wx >> l) & 1) ex.v[l] = vx.v[l];
-        if ((wy >> l) & 1) ey.v[l] = vy.v[l];
-        if ((wz >> l) & 1) ez.v[l] = vz.v[l];
-        check += ex.v[l] + ey.v[l] + ez.v[l];
-      }
-      if (wx) stv(s.E[0] + b, ex);
-      if (wy) stv(s.E[1] + b, ey);
-      if (wz) stv(s.E[2] + b, ez);
+    for (int l = 0; l < N; l++) {
+      if ((onx >> l) & 1) ex.v[l] = vx.v[l];
+      if ((onyz >> l) & 1) { ey.v[l] = vy.v[l]; ez.v[l] = vz.v[l]; }
+    }
+    if (!(mx | my | mz)) {
+      if (upx) { stv(s.E[0] + b, ex); check += sum(ex); }
+      if (upy) { stv(s.E[1] + b, ey); check += sum(ey); }
+      if (upz) { stv(s.E[2] + b, ez); check += sum(ez); }
     } else {
 #pragma unroll
       for (int l = 0; l < N; l++) {
-        if ((wx >> l) & 1) { s.E[0][b + l] = vx.v[l]; check += vx.v[l]; }
-        if ((wy >> l) & 1) { s.E[1][b + l] = vy.v[l]; check += vy.v[l]; }
-        if ((wz >> l) & 1) { s.E[2][b + l] = vz.v[l]; check += vz.v[l]; }
+        if (upx && !((mx >> l) & 1)) { s.E[0][b + l] = ex.v[l]; check += ex.v[l]; }
+        if (upy && !((my >> l) & 1)) { s.E[1][b + l] = ey.v[l]; check += ey.v[l]; }
+        if (upz && !((mz >> l) & 1)) { s.E[2][b + l] = ez.v[l]; check += ez.v[l]; }
       }
     }
     hxm = hx;
