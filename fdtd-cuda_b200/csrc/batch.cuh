@@ -3,23 +3,22 @@
 // builds allow one trial, main.cu:2386-2389).
 //
 // Every member is an ordinary fdtd_sim (its own fields, tables, DFT and
-// clock); the batch adds, in device memory, one descriptor per member and
-// one list of (member, tile) work items for the Yee passes.  A time step of
-// the whole batch is
-//   h_pass_batch      two persistent grids: the CPML-free tiles of all
-//                     members from one queue, the CPML edge tiles from another
-//   line_step         one launch, one CTA per member (double-buffered line E)
-//   tfsf_apply        both TFSF halves, one launch, blockIdx.y = member
-//   (hydrodynamic members: their three dispersive kernels, per member)
-//   e_pass_batch      two persistent grids as for H
-//   metal_e           one launch
+// clock); the batch adds, in device memory, one descriptor per member and the
+// block lists of its two launches per time step.  A block of a list is the line
+// step of a member, a share of its dispersive cells, or vectors and planes of
+// its grid (the direct passes, flat.cuh):
+//   h_flat_batch      line steps, hydrodynamic currents, H pass
+//   tfsf_apply_batch  only with members at oblique incidence
+//   e_flat_batch      dispersive cells, E pass
 //   dft_sample        one launch every dft_every steps, blockIdx.z = member
 //   the DFT contraction (job, phasors, product, reset), one launch each,
 //                     every 32 samples; it contracts each member's first
 //                     ring half once that holds 64 samples
 // so the launch count per step does not grow with the member count, and
 // small members that could not fill the GPU alone share it.  Runs of
-// 32 * dft_every steps are captured into one CUDA graph and replayed.
+// 32 * dft_every steps are captured into one CUDA graph and replayed.  A batch
+// with a member that the direct passes do not take (the staged ones are forced,
+// or it is beyond their 32-bit offsets) steps its members one after another.
 //
 // This file is included at the end of fdtd.cu (it uses the simulation
 // internals defined there).
@@ -32,7 +31,6 @@ struct BatchSim {
   MetalView<T> m;
   LineArgs line;
   DftView dft;
-  ShellCells sh_h, sh_e;
   TfsfTable tf_h, tf_e;
   T* ring;
   double2* tw;
@@ -45,18 +43,59 @@ __global__ void tfsf_apply_batch(const BatchSim<T>* __restrict__ b) {
   const BatchSim<T>& x = b[blockIdx.y];
   tfsf_apply_body(x.v, x.tf_h, x.tf_e, x.line);
 }
+
+// A block of a batch launch: (member | role << 20, first vector's block or the
+// block of the role, first plane, planes per thread | z groups << 16).  A grid
+// block's 256 threads are z groups of 256 / groups vectors each, one above the
+// other.
+enum { kItemGrid = 0, kItemLine = 1, kItemCells = 2 };
+
+// The member's view in shared memory: the passes read it where a single
+// simulation's kernel reads its parameters.
 template <typename T>
-__global__ void __launch_bounds__(1024) line_step_batch(const BatchSim<T>* __restrict__ b) {
-  const BatchSim<T>& x = b[blockIdx.y];
-  const int t = x.clk->t;
+__device__ __forceinline__ void batch_view(SimView<T>& dst, const SimView<T>& src) {
+  static_assert(sizeof(SimView<T>) % 8 == 0, "copied in 8-byte words");
+  const unsigned long long* p = reinterpret_cast<const unsigned long long*>(&src);
+  unsigned long long* q = reinterpret_cast<unsigned long long*>(&dst);
+  for (int w = threadIdx.x; w < (int)(sizeof(SimView<T>) / 8); w += kFlatThreads) q[w] = __ldg(p + w);
   __syncthreads();
-  line_step_body(x.line, x.v, x.probe_id, t);
-  if (threadIdx.x == 0) x.clk->th = t + 1;
 }
-template <typename T>
-__global__ void metal_e_batch(const BatchSim<T>* __restrict__ b) {
-  const BatchSim<T>& x = b[blockIdx.y];
-  metal_e_cell(x.v, x.m, x.clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+
+template <typename T, bool RING, bool HYDRO>
+__global__ void __launch_bounds__(kFlatThreads, 2)
+    h_flat_batch(const BatchSim<T>* __restrict__ b, const int4* __restrict__ items) {
+  __shared__ SimView<T> s;
+  const int4 it = items[blockIdx.x];
+  const BatchSim<T>& x = b[it.x & 0xFFFFF];
+  const int role = it.x >> 20;
+  if (role == kItemLine) {
+    line_step_body(x.line, x.v, x.probe_id, x.clk->th);
+    return;
+  }
+  if (HYDRO && role == kItemCells) {
+    hydro_p_any(x.v, x.m, x.clk->th, it.y * kFlatThreads + (int)threadIdx.x);
+    return;
+  }
+  batch_view(s, x.v);
+  const int kz = it.w & 0xFFFF, vx = kFlatThreads / (it.w >> 16), tz = threadIdx.x / vx;
+  h_flat_cells<T, RING, true>(s, (unsigned)(it.y * vx + (threadIdx.x - tz * vx)), it.z + tz * kz, kz);
+}
+template <typename T, bool RING, bool HYDRO>
+__global__ void __launch_bounds__(kFlatThreads, 2)
+    e_flat_batch(const BatchSim<T>* __restrict__ b, const int4* __restrict__ items) {
+  __shared__ SimView<T> s;
+  const int4 it = items[blockIdx.x];
+  const BatchSim<T>& x = b[it.x & 0xFFFFF];
+  if ((it.x >> 20) == kItemCells) {
+    const int q = it.y * kFlatThreads + (int)threadIdx.x, t = x.clk->t - 1;
+    if (HYDRO) hydro_e_any(x.v, x.m, t, q);
+    else metal_e_cell(x.v, x.m, t, q);
+    return;
+  }
+  if (it.y == 0 && it.z == 0 && threadIdx.x == 0) x.clk->th = x.clk->t;
+  batch_view(s, x.v);
+  const int kz = it.w & 0xFFFF, vx = kFlatThreads / (it.w >> 16), tz = threadIdx.x / vx;
+  e_flat_cells<T, RING, true>(s, (unsigned)(it.y * vx + (threadIdx.x - tz * vx)), it.z + tz * kz, kz);
 }
 template <typename T>
 __global__ void dft_sample_batch(const BatchSim<T>* __restrict__ b) {
@@ -90,16 +129,6 @@ __global__ void dft_job_done_batch(const BatchSim<T>* __restrict__ b) {
 
 }  // namespace fdtd
 
-// Pass launch shapes of the batch.  Work items are 32 x 4 tiles (TY = 4 for
-// every launch, so that the CPML-edge and CPML-free item lists partition
-// the cells); each size bucket of members has its own z-chunk, carried by
-// its items; the edge and the interior launch of each pass have their own
-// kernel variant (register cap MINB and ring depth S).  fdtd_batch_create
-// times the choices (batch_tune).
-constexpr int kBatchTY = 4;
-#define FDTD_BATCH_VARIANTS(X) X(1, 4) X(6, 4) X(8, 4) X(6, 6)
-constexpr int kBatchVariants = 4;
-static const int kBatchVar[kBatchVariants][2] = {{1, 4}, {6, 4}, {8, 4}, {6, 6}};  // (MINB, S)
 constexpr int kBatchBucket = 16;  // members bucketed by their largest edge, 16 cells a bucket
 constexpr int kBatchMaxBuckets = FDTD_BATCH_MAX_BUCKETS;
 
@@ -109,23 +138,21 @@ struct fdtd_batch {
   std::vector<std::unique_ptr<fdtd_sim>> sims;
   std::vector<std::unique_ptr<DevBuf>> bufs;
   void* descs = nullptr;  // BatchSim<T>[n]
-  void* views = nullptr;  // SimView<T>[n]
-  int4* items = nullptr;  // (member | z-chunk << 20, bx, by, bz): edge items, then interior items
-  int* queue = nullptr;   // [4] work counters: H edge, H interior, E edge, E interior
-  int nedge = 0, ninner = 0;
-  size_t items_cap = 0;
-  // size buckets and the z-chunk of each; member -> bucket
+  // block lists of the two launches (H, E), kept and grown: the graph of the
+  // step holds their addresses
+  int4* items[2] = {nullptr, nullptr};
+  int nitems[2] = {0, 0};
+  size_t items_cap[2] = {0, 0};
+  bool direct = true;  // every member takes the direct passes
+  bool ring = false;   // their planes are copied ahead
+  // size buckets and their planes per thread; member -> bucket
   int nbuckets = 0;
-  int bucket_lo[kBatchMaxBuckets] = {}, bucket_members[kBatchMaxBuckets] = {}, bucket_kc[kBatchMaxBuckets] = {};
+  int bucket_lo[kBatchMaxBuckets] = {}, bucket_members[kBatchMaxBuckets] = {}, bucket_kz[kBatchMaxBuckets] = {};
   float bucket_ms[kBatchMaxBuckets] = {};
   std::vector<int> member_bucket;
-  // kernel variant (index into kBatchVar) and persistent grid per launch:
-  // [pass H / E][edge / interior]
-  int var[2][2] = {{1, 1}, {1, 1}};
-  int grid[2][2] = {{0, 0}, {0, 0}};
   int sms = 0;
   bool tuned = false;
-  unsigned g_f = 0, g_m = 0, g_s = 0, g_tw = 0, g_c = 0;
+  unsigned g_f = 0, g_s = 0, g_tw = 0, g_c = 0;
   int t = 0, host_nsamp = 0, dft_every = 0, tend = 0;
   long long kernels = 0, graph_launches = 0, graph_kernels = 0;
   cudaGraphExec_t graph = nullptr;
@@ -146,32 +173,23 @@ struct fdtd_batch {
   }
 };
 
-// Work items of member i with z-chunk kc: the tiles that touch no CPML slab
-// go to `inner` (the rule of build_tiles), the others to `edge`.
-static void batch_member_items(const fdtd_sim* s, int i, int kc, std::vector<int4>& edge, std::vector<int4>& inner) {
-  const int nbx = (s->NX + 31) / 32, nby = (s->NY + kBatchTY - 1) / kBatchTY, nbz = (s->NZ + kc - 1) / kc;
-  const int nb3[3] = {nbx, nby, nbz}, w3[3] = {32, kBatchTY, kc};
-  int lo[3], hi[3];
-  for (int a = 0; a < 3; a++) {
-    const int Nc = s->su.Nc[a], F = s->su.F[a];
-    lo[a] = (Nc + 1 + w3[a] - 1) / w3[a];
-    hi[a] = std::min(F >= w3[a] ? (F - w3[a]) / w3[a] + 1 : 0, nb3[a]);
-  }
-  const int tag = i | (kc << 20);
-  for (int bz = 0; bz < nbz; bz++)
-    for (int by = 0; by < nby; by++)
-      for (int bx = 0; bx < nbx; bx++) {
-        const bool in = bx >= lo[0] && bx < hi[0] && by >= lo[1] && by < hi[1] && bz >= lo[2] && bz < hi[2];
-        (in ? inner : edge).push_back(make_int4(tag, bx, by, bz));
-      }
+// Planes per thread as blocks: a block spans 8, 16 or 32 planes (its z-chunk),
+// short runs of planes as groups of threads above one another.
+static int batch_kchunk(int kz) { return std::max(8, kz); }
+
+// The grid blocks of member i with kz planes per thread.
+template <typename T>
+static void batch_member_items(const fdtd_sim* s, int i, int kz, std::vector<int4>& out) {
+  const int kc = batch_kchunk(kz), groups = kc / kz, vx = kFlatThreads / groups;
+  const int nv = (int)(s->plane / Vec<T>::N), nx = (nv + vx - 1) / vx;
+  for (int k = 0; k < s->NZ; k += kc)
+    for (int x = 0; x < nx; x++) out.push_back(make_int4(i, x, k, kz | groups << 16));
 }
 
 template <typename T>
 static fdtd_status batch_build(fdtd_batch* b) {
   const int n = (int)b->sims.size();
   std::vector<BatchSim<T>> d(n);
-  std::vector<SimView<T>> v(n);
-  std::vector<int4> items, inner;
   for (int i = 0; i < n; i++) {
     fdtd_sim* s = b->sims[i].get();
     BatchSim<T>& x = d[i];
@@ -179,18 +197,17 @@ static fdtd_status batch_build(fdtd_batch* b) {
     x.m = mview<T>(s);
     x.line = s->line;
     x.dft = s->dft;
-    x.sh_h = s->shell_h;
-    x.sh_e = s->shell_e;
-    x.tf_h = s->tf_h;
-    x.tf_e = s->tf_e;
+    if (!s->fused_tfsf) {  // else the passes apply the corrections
+      x.tf_h = s->tf_h;
+      x.tf_e = s->tf_e;
+    }
+    b->direct = b->direct && s->hcfg.kz > 0;
     x.ring = static_cast<T*>(s->ring);
     x.tw = s->twiddles;
     x.clk = s->clk;
     x.probe_id = s->probe_id;
-    v[i] = x.v;
     auto blocks = [](long long cells, int per) { return (unsigned)((cells + per - 1) / per); };
-    b->g_f = std::max(b->g_f, blocks((long long)s->tf_h.n + s->tf_e.n, 256));
-    b->g_m = std::max(b->g_m, blocks((long long)s->nmetal[0] + s->nmetal[1] + s->nmetal[2], 128));
+    b->g_f = std::max(b->g_f, blocks((long long)x.tf_h.n + x.tf_e.n, 256));
     int maxn = 0;
     for (int f = 0; f < 12; f++) maxn = std::max(maxn, s->dft.face[f].na * s->dft.face[f].nb);
     b->g_s = std::max(b->g_s, blocks(maxn, 256));
@@ -198,15 +215,10 @@ static fdtd_status batch_build(fdtd_batch* b) {
     b->g_c = std::max(b->g_c, (unsigned)(s->dft.rows / kDftRows));
   }
   BatchSim<T>* dd;
-  SimView<T>* dv;
   CUDA_TRY(b->alloc(&dd, n));
-  CUDA_TRY(b->alloc(&dv, n));
-  CUDA_TRY(b->alloc(&b->queue, 4));
   CUDA_TRY(cudaMemcpy(dd, d.data(), n * sizeof(BatchSim<T>), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dv, v.data(), n * sizeof(SimView<T>), cudaMemcpyHostToDevice));
   b->descs = dd;
-  b->views = dv;
-  // size buckets by the largest edge, z-chunk 16 until tuned
+  // size buckets by the largest edge
   b->member_bucket.assign(n, 0);
   std::vector<int> key(n);
   for (int i = 0; i < n; i++) {
@@ -222,7 +234,7 @@ static fdtd_status batch_build(fdtd_batch* b) {
   b->nbuckets = (int)keys.size();
   for (int q = 0; q < b->nbuckets; q++) {
     b->bucket_lo[q] = keys[q] * kBatchBucket + 1;
-    b->bucket_kc[q] = 16;
+    b->bucket_kz[q] = 8;
     b->bucket_members[q] = 0;
   }
   for (int i = 0; i < n; i++) {
@@ -232,132 +244,84 @@ static fdtd_status batch_build(fdtd_batch* b) {
     b->bucket_members[q]++;
   }
   CUDA_TRY(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
-  // every batch pass variant may take more than 48 KB of shared memory
-#define FDTD_BATCH_ATTR(MB, S)                                                                                  \
-  CUDA_TRY(cudaFuncSetAttribute(h_pass_batch<T, kBatchTY, S, MB, true>,                                         \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged_smem<T, kBatchTY, S>())); \
-  CUDA_TRY(cudaFuncSetAttribute(h_pass_batch<T, kBatchTY, S, MB, false>,                                        \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged_smem<T, kBatchTY, S>())); \
-  CUDA_TRY(cudaFuncSetAttribute(e_pass_batch<T, kBatchTY, S, MB, true>,                                         \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged_smem<T, kBatchTY, S>())); \
-  CUDA_TRY(cudaFuncSetAttribute(e_pass_batch<T, kBatchTY, S, MB, false>,                                        \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged_smem<T, kBatchTY, S>()));
-  FDTD_BATCH_VARIANTS(FDTD_BATCH_ATTR)
-#undef FDTD_BATCH_ATTR
+  {
+    const void* k[4] = {(const void*)h_flat_batch<T, true, false>, (const void*)h_flat_batch<T, true, true>,
+                        (const void*)e_flat_batch<T, true, false>, (const void*)e_flat_batch<T, true, true>};
+    for (const void* f : k)
+      CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatRingBytes));
+  }
   CUDA_TRY(cudaFuncSetAttribute(dft_contract_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)dft_smem_bytes<T>()));
   return FDTD_OK;
 }
 
-// Persistent grid of one pass launch: every CTA slot of the GPU once.
-template <typename T, bool EPASS, bool PML>
-static int batch_grid(fdtd_batch* b, int var) {
-  int per = 0;
-  const int mb = kBatchVar[var][0], sg = kBatchVar[var][1];
-#define FDTD_BATCH_OCC(MB, S)                                                                                   \
-  if (mb == MB && sg == S) {                                                                                     \
-    if (EPASS)                                                                                                  \
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, e_pass_batch<T, kBatchTY, S, MB, PML>, 32 * kBatchTY,  \
-                                                    staged_smem<T, kBatchTY, S>());                             \
-    else                                                                                                        \
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, h_pass_batch<T, kBatchTY, S, MB, PML>, 32 * kBatchTY,  \
-                                                    staged_smem<T, kBatchTY, S>());                             \
-  }
-  FDTD_BATCH_VARIANTS(FDTD_BATCH_OCC)
-#undef FDTD_BATCH_OCC
-  return std::max(1, per) * b->sms;
-}
-
-// The item lists for the current per-bucket z-chunks, uploaded (edge items
-// first, then interior items).
-static fdtd_status batch_upload_items(fdtd_batch* b, const std::vector<int>* only_bucket_members = nullptr) {
-  std::vector<int4> edge, inner;
+// The block lists for the current planes per thread, uploaded.  only: a bucket,
+// or -1 for all of them; grid: the grid blocks alone (for timing).
+template <typename T>
+static fdtd_status batch_upload_items(fdtd_batch* b, int only = -1, bool grid = false) {
   const int n = (int)b->sims.size();
-  for (int i = 0; i < n; i++) {
-    if (only_bucket_members && std::find(only_bucket_members->begin(), only_bucket_members->end(), i) ==
-                                   only_bucket_members->end())
-      continue;
-    batch_member_items(b->sims[i].get(), i, b->bucket_kc[b->member_bucket[i]], edge, inner);
+  for (int p = 0; p < 2; p++) {
+    std::vector<int4> v;
+    if (!grid && p == 0)
+      for (int i = 0; i < n; i++) v.push_back(make_int4(i | kItemLine << 20, 0, 0, 0));
+    if (!grid && (p == 1 || b->hydro))
+      for (int i = 0; i < n; i++) {
+        const fdtd_sim* s = b->sims[i].get();
+        const int nb = (s->nmetal[0] + s->nmetal[1] + s->nmetal[2] + kFlatThreads - 1) / kFlatThreads;
+        for (int q = 0; q < nb; q++) v.push_back(make_int4(i | kItemCells << 20, q, 0, 0));
+      }
+    for (int i = 0; i < n; i++)
+      if (only < 0 || b->member_bucket[i] == only)
+        batch_member_items<T>(b->sims[i].get(), i, b->bucket_kz[b->member_bucket[i]], v);
+    b->nitems[p] = (int)v.size();
+    if (v.empty()) continue;
+    if (!b->items[p] || b->items_cap[p] < v.size()) {
+      int4* d;
+      CUDA_TRY(b->alloc(&d, v.size()));
+      b->items[p] = d;
+      b->items_cap[p] = v.size();
+    }
+    CUDA_TRY(cudaMemcpy(b->items[p], v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
   }
-  b->nedge = (int)edge.size();
-  b->ninner = (int)inner.size();
-  edge.insert(edge.end(), inner.begin(), inner.end());
-  if (edge.empty()) return FDTD_OK;
-  // one buffer, kept and grown: the graph of the step holds its address
-  static_assert(sizeof(int4) == 16, "int4 items");
-  if (!b->items || b->items_cap < edge.size()) {
-    int4* d;
-    CUDA_TRY(b->alloc(&d, edge.size()));
-    b->items = d;
-    b->items_cap = edge.size();
-  }
-  CUDA_TRY(cudaMemcpy(b->items, edge.data(), edge.size() * sizeof(int4), cudaMemcpyHostToDevice));
   return FDTD_OK;
 }
 
-// One persistent pass launch of variant `var` over items [off, off + n),
-// counting its work from queue; pdl = a programmatic dependency on the
-// launch before it on the stream.
-template <typename T, bool EPASS, bool PML>
-static void batch_pass_launch(fdtd_batch* b, int var, int grid, int off, int n, int* queue, cudaStream_t st,
-                              bool pdl) {
-  const SimView<T>* v = static_cast<const SimView<T>*>(b->views);
-  const int4* items = b->items + off;
-  const int mb = kBatchVar[var][0], sg = kBatchVar[var][1];
-#define FDTD_BATCH_LAUNCH(MB, S)                                                                              \
-  if (mb == MB && sg == S) {                                                                                   \
-    const size_t smem = staged_smem<T, kBatchTY, S>();                                                        \
-    if (EPASS) {                                                                                              \
-      if (pdl) launch_ex(true, e_pass_batch<T, kBatchTY, S, MB, PML>, dim3(grid), dim3(32, kBatchTY), smem,  \
-                                st, v, items, n, queue);                                                      \
-      else e_pass_batch<T, kBatchTY, S, MB, PML><<<grid, dim3(32, kBatchTY), smem, st>>>(v, items, n, queue); \
-    } else {                                                                                                  \
-      if (pdl) launch_ex(true, h_pass_batch<T, kBatchTY, S, MB, PML>, dim3(grid), dim3(32, kBatchTY), smem,  \
-                                st, v, items, n, queue);                                                      \
-      else h_pass_batch<T, kBatchTY, S, MB, PML><<<grid, dim3(32, kBatchTY), smem, st>>>(v, items, n, queue); \
-    }                                                                                                         \
-  }
-  FDTD_BATCH_VARIANTS(FDTD_BATCH_LAUNCH)
-#undef FDTD_BATCH_LAUNCH
+template <typename T, bool RING, bool HYDRO>
+static void batch_launch_form(fdtd_batch* b, int p, cudaStream_t st) {
+  const BatchSim<T>* d = static_cast<const BatchSim<T>*>(b->descs);
+  const dim3 g(b->nitems[p]), blk(kFlatThreads);
+  const size_t smem = RING ? kFlatRingBytes : 0;
+  if (p == 0) h_flat_batch<T, RING, HYDRO><<<g, blk, smem, st>>>(d, b->items[0]);
+  else e_flat_batch<T, RING, HYDRO><<<g, blk, smem, st>>>(d, b->items[1]);
 }
-
-// One pass of every member: the CPML edge items, then the CPML-free items
-// with a programmatic dependency (they touch disjoint cells); returns the
-// number of launches.
-template <typename T, bool EPASS>
-static int batch_pass(fdtd_batch* b, int* queue, cudaStream_t st) {
-  const int p = EPASS ? 1 : 0;
-  int k = 0;
-  if (b->nedge) {
-    batch_pass_launch<T, EPASS, true>(b, b->var[p][0], b->grid[p][0], 0, b->nedge, queue, st, false);
-    k++;
+template <typename T>
+static void batch_launch(fdtd_batch* b, int p, cudaStream_t st) {
+  if (b->ring) {
+    if (b->hydro) batch_launch_form<T, true, true>(b, p, st);
+    else batch_launch_form<T, true, false>(b, p, st);
+  } else {
+    if (b->hydro) batch_launch_form<T, false, true>(b, p, st);
+    else batch_launch_form<T, false, false>(b, p, st);
   }
-  if (b->ninner) {
-    batch_pass_launch<T, EPASS, false>(b, b->var[p][1], b->grid[p][1], b->nedge, b->ninner, queue + 1, st, true);
-    k++;
-  }
-  return k;
 }
 
 template <typename T>
 static void batch_enqueue_step(fdtd_batch* b, cudaStream_t st) {
-  const int n = (int)b->sims.size();
-  const BatchSim<T>* d = static_cast<const BatchSim<T>*>(b->descs);
-  cudaMemsetAsync(b->queue, 0, 4 * sizeof(int), st);
-  int k = batch_pass<T, false>(b, b->queue, st);
-  // the line step writes the line's other E buffer, so the fused TFSF launch
-  // after it still applies the H half with the line's E from before it
-  line_step_batch<T><<<dim3(1, n), 1024, 0, st>>>(d);
-  k++;
-  if (b->g_f) { tfsf_apply_batch<T><<<dim3(b->g_f, n), 256, 0, st>>>(d); k++; }
-  if (b->hydro)
+  if (!b->direct) {
     for (auto& s : b->sims) {
       const long long k0 = s->kernels;
-      launch_metal<T>(s.get(), st);  // UpdateHydroP* read E^n here
-      k += (int)(s->kernels - k0);
+      enqueue_step<T>(s.get(), st);
+      b->kernels += s->kernels - k0;
     }
-  k += batch_pass<T, true>(b, b->queue + 2, st);
-  if (!b->hydro && b->g_m) { metal_e_batch<T><<<dim3(b->g_m, n), 128, 0, st>>>(d); k++; }
+    b->t++;
+    return;
+  }
+  const int n = (int)b->sims.size();
+  const BatchSim<T>* d = static_cast<const BatchSim<T>*>(b->descs);
+  int k = 2;
+  batch_launch<T>(b, 0, st);
+  if (b->g_f) { tfsf_apply_batch<T><<<dim3(b->g_f, n), 256, 0, st>>>(d); k++; }
+  batch_launch<T>(b, 1, st);
   if (b->dft_every > 0 && b->t % b->dft_every == 0) {
     dft_sample_batch<T><<<dim3(b->g_s, 12, n), 256, 0, st>>>(d);
     k++;
@@ -375,18 +339,17 @@ static void batch_enqueue_step(fdtd_batch* b, cudaStream_t st) {
   b->t++;
 }
 
-// Mean device time of `reps` runs of both passes (H and E, each its edge
-// and interior launch) over the current item lists, after one untimed run.
-// On the zero state the passes leave the fields at zero.
+// Mean device time of `reps` runs of both passes over the current block lists
+// (grid blocks), after one untimed run.  On the zero state the passes leave the
+// fields at zero.
 template <typename T>
 static fdtd_status batch_time_passes(fdtd_batch* b, int reps, float* ms) {
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
   auto go = [&]() {
-    cudaMemsetAsync(b->queue, 0, 4 * sizeof(int), 0);
-    batch_pass<T, false>(b, b->queue, 0);
-    batch_pass<T, true>(b, b->queue + 2, 0);
+    batch_launch<T>(b, 0, 0);
+    batch_launch<T>(b, 1, 0);
   };
   go();
   cudaEventRecord(e0, 0);
@@ -402,64 +365,57 @@ static fdtd_status batch_time_passes(fdtd_batch* b, int reps, float* ms) {
   return FDTD_OK;
 }
 
-// The autotuner of the batch's passes (no counterpart in the reference):
-// per size bucket the z-chunk (8, 16 or 32 planes) with the bucket's
-// members alone, then per launch (H / E pass, edge / interior items) the
-// kernel variant over the whole batch.  FDTD_TUNE=0, or a batch under 2^20
-// cells, keeps z-chunk 16 and variant (MINB 6, S 4) everywhere.
+// The autotuner of the batch's passes (no counterpart in the reference): per
+// size bucket the planes per thread (2, 4, 8 or 16) with the bucket's members
+// alone, then the same number for every bucket over the whole batch: members
+// alone want short runs, which fill the GPU, a full batch longer ones, which
+// re-read less.  FDTD_TUNE=0, or a batch under 2^20 cells, takes the most
+// planes, up to 8, that leave two blocks a multiprocessor.
 template <typename T>
 static fdtd_status batch_tune(fdtd_batch* b) {
-  for (int p = 0; p < 2; p++)
-    for (int q = 0; q < 2; q++) b->var[p][q] = 1;
-  auto grids = [&]() {
-    b->grid[0][0] = batch_grid<T, false, true>(b, b->var[0][0]);
-    b->grid[0][1] = batch_grid<T, false, false>(b, b->var[0][1]);
-    b->grid[1][0] = batch_grid<T, true, true>(b, b->var[1][0]);
-    b->grid[1][1] = batch_grid<T, true, false>(b, b->var[1][1]);
-  };
-  grids();
-  long long cells = 0;
-  for (const auto& s : b->sims) cells += s->ncell;
+  if (!b->direct) return FDTD_OK;
+  long long cells = 0, vecs = 0;
+  for (const auto& s : b->sims) {
+    cells += s->ncell;
+    vecs += (long long)(s->ncell / Vec<T>::N);
+  }
+  int kz = 1;
+  while (kz < 8 && vecs / (2 * kz * kFlatThreads) >= 2LL * b->sms) kz *= 2;
+  for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = kz;
   const char* env = std::getenv("FDTD_TUNE");
   fdtd_status st;
-  if ((env && env[0] == '0') || cells < (1LL << 20)) return batch_upload_items(b);
-  const int n = (int)b->sims.size();
-  // z-chunk per bucket, its members alone
+  if ((env && env[0] == '0') || cells < (1LL << 20)) return batch_upload_items<T>(b);
+  std::vector<int> chosen(b->nbuckets, kz);
+  float ms;
   for (int q = 0; q < b->nbuckets; q++) {
-    std::vector<int> mem;
-    for (int i = 0; i < n; i++)
-      if (b->member_bucket[i] == q) mem.push_back(i);
     float best = 1e30f;
-    int best_kc = 16;
-    for (int kc : {8, 16, 32}) {
-      b->bucket_kc[q] = kc;
-      if ((st = batch_upload_items(b, &mem)) != FDTD_OK) return st;
-      float ms;
+    for (int z : {2, 4, 8, 16}) {
+      b->bucket_kz[q] = z;
+      if ((st = batch_upload_items<T>(b, q, true)) != FDTD_OK) return st;
       if ((st = batch_time_passes<T>(b, 3, &ms)) != FDTD_OK) return st;
-      if (ms < best) { best = ms; best_kc = kc; }
+      if (ms < best) { best = ms; chosen[q] = z; }
     }
-    b->bucket_kc[q] = best_kc;
     b->bucket_ms[q] = best;
   }
-  if ((st = batch_upload_items(b)) != FDTD_OK) return st;
-  // the variant of each launch, the others held
-  for (int p = 0; p < 2; p++)
-    for (int e = 0; e < 2; e++) {
-      float best = 1e30f;
-      int best_v = b->var[p][e];
-      for (int v = 0; v < kBatchVariants; v++) {
-        b->var[p][e] = v;
-        grids();
-        float ms;
-        if ((st = batch_time_passes<T>(b, 3, &ms)) != FDTD_OK) return st;
-        if (ms < best) { best = ms; best_v = v; }
-      }
-      b->var[p][e] = best_v;
-      grids();
+  // -1: each bucket's own; with and without the ring
+  float best = 1e30f;
+  int best_z = -1;
+  bool best_ring = false;
+  for (int z : {-1, 4, 8, 16, 32}) {
+    for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = z < 0 ? chosen[q] : z;
+    if ((st = batch_upload_items<T>(b, -1, true)) != FDTD_OK) return st;
+    for (int ring = 0; ring < 2; ring++) {
+      if (ring ? z >= 0 && z < 8 : z == 32) continue;
+      b->ring = ring;
+      if ((st = batch_time_passes<T>(b, 3, &ms)) != FDTD_OK) return st;
+      if (ms < best) { best = ms; best_z = z; best_ring = ring; }
     }
+  }
+  for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = best_z < 0 ? chosen[q] : best_z;
+  b->ring = best_ring;
   b->tuned = true;
   CUDA_TRY(cudaGetLastError());
-  return FDTD_OK;
+  return batch_upload_items<T>(b);
 }
 
 template <typename T>
@@ -468,7 +424,7 @@ static fdtd_status batch_step(fdtd_batch* b, int nsteps, cudaStream_t st) {
   const int G = every * kSampleBlock;
   int done = 0;
   while (done < nsteps) {
-    const bool aligned = b->t % G == 0 && b->host_nsamp == 0 && nsteps - done >= G;
+    const bool aligned = b->direct && b->t % G == 0 && b->host_nsamp == 0 && nsteps - done >= G;
     if (aligned) {
       if (!b->graph) {
         if (!b->cap) CUDA_TRY(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
@@ -498,8 +454,10 @@ static fdtd_status batch_step(fdtd_batch* b, int nsteps, cudaStream_t st) {
   }
   // the members' host mirrors follow the batch clock
   for (auto& s : b->sims) {
-    s->t = b->t;
-    s->host_nsamp = b->host_nsamp;
+    if (b->direct) {
+      s->t = b->t;
+      s->host_nsamp = b->host_nsamp;
+    }
     s->steps_done += nsteps;
   }
   CUDA_TRY(cudaGetLastError());
@@ -586,15 +544,15 @@ extern "C" fdtd_status fdtd_batch_get_tuning(const fdtd_batch* b, fdtd_batch_tun
     out->edge_lo[q] = b->bucket_lo[q];
     out->edge_hi[q] = q + 1 < b->nbuckets ? b->bucket_lo[q + 1] - 1 : INT_MAX;
     out->members[q] = b->bucket_members[q];
-    out->kchunk[q] = b->bucket_kc[q];
+    out->kchunk[q] = batch_kchunk(b->bucket_kz[q]);
     out->bucket_ms[q] = b->bucket_ms[q];
   }
   out->tile_x = 32;
-  out->tile_y = kBatchTY;
+  out->tile_y = b->fp64 ? Vec<double>::N : Vec<float>::N;
   for (int p = 0; p < 2; p++)
     for (int e = 0; e < 2; e++) {
-      out->minb[p][e] = kBatchVar[b->var[p][e]][0];
-      out->stages[p][e] = kBatchVar[b->var[p][e]][1];
+      out->minb[p][e] = 2;
+      out->stages[p][e] = b->ring ? kFlatRing : 1;
     }
   return FDTD_OK;
 }

@@ -873,7 +873,7 @@ static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out,
   // face, component and z index alone (normal incidence): the line step then
   // evaluates a few hundred increments a step.  Oblique incidence has nearly as
   // many distinct corrections as face cells and keeps the TFSF launch.
-  s->fused_tfsf = direct_passes(s.get()) && s->inc_ok && tune && s->ncell < fuse_tfsf_below(s->fp64);
+  s->fused_tfsf = direct_passes(s.get()) && s->inc_ok && s->ncell < fuse_tfsf_below(s->fp64);
   if (s->fused_tfsf) {
     st = s->fp64 ? fuse_tfsf<double>(s.get()) : fuse_tfsf<float>(s.get());
     if (st != FDTD_OK) return st;

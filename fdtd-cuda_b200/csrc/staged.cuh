@@ -537,30 +537,6 @@ __global__ void __launch_bounds__(32 * TY, MINB) h_pass_t(const __grid_constant_
   pdl_wait();
 }
 
-// Batched form: a persistent grid that takes (simulation, tile) work items
-// from a queue shared by every simulation of a batch; the views live in
-// device memory, one per simulation, and every item carries the z-chunk of
-// its simulation's size bucket.
-template <typename T, int TY, int S, int MINB, bool PML>
-__global__ void __launch_bounds__(32 * TY, MINB) h_pass_batch(const SimView<T>* __restrict__ views,
-                                                           const int4* __restrict__ items, int nitems,
-                                                           int* __restrict__ queue) {
-  __shared__ int next;
-  pdl_launch_dependents();  // the second launch of the pass may fill this one's tail
-  for (;;) {
-    __syncthreads();  // the previous item is finished with the stage ring and with next
-    if (threadIdx.x == 0 && threadIdx.y == 0) next = atomicAdd(queue, 1);
-    __syncthreads();
-    const int it = next;
-    if (it >= nitems) {
-      pdl_wait();
-      return;
-    }
-    const int4 w = items[it];  // (simulation | z-chunk << 20, bx, by, bz)
-    h_pass_tile<T, TY, S, PML>(views[w.x & 0xFFFFF], w.x >> 20, w.y, w.z, w.w);
-  }
-}
-
 // ---------------------------------------------------------------------
 // E pass (UPDATE_ex/ey/ez, main.cu:1048-1912).
 // Needs H at k and k-1 (halo family, one row/column of -1 halo) and E at k
@@ -776,30 +752,6 @@ __global__ void __launch_bounds__(32 * TY, MINB) e_pass_t(const __grid_constant_
   tile_of(tm, bx, by, bz);
   e_pass_tile<T, TY, S, PML, true>(s, kchunk, bx, by, bz, &maps);
   pdl_wait();
-}
-
-// Batched form: a persistent grid that takes (simulation, tile) work items
-// from a queue shared by every simulation of a batch; the views live in
-// device memory, one per simulation, and every item carries the z-chunk of
-// its simulation's size bucket.
-template <typename T, int TY, int S, int MINB, bool PML>
-__global__ void __launch_bounds__(32 * TY, MINB) e_pass_batch(const SimView<T>* __restrict__ views,
-                                                           const int4* __restrict__ items, int nitems,
-                                                           int* __restrict__ queue) {
-  __shared__ int next;
-  pdl_launch_dependents();  // the second launch of the pass may fill this one's tail
-  for (;;) {
-    __syncthreads();  // the previous item is finished with the stage ring and with next
-    if (threadIdx.x == 0 && threadIdx.y == 0) next = atomicAdd(queue, 1);
-    __syncthreads();
-    const int it = next;
-    if (it >= nitems) {
-      pdl_wait();
-      return;
-    }
-    const int4 w = items[it];  // (simulation | z-chunk << 20, bx, by, bz)
-    e_pass_tile<T, TY, S, PML>(views[w.x & 0xFFFFF], w.x >> 20, w.y, w.z, w.w);
-  }
 }
 
 }  // namespace fdtd

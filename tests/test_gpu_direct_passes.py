@@ -106,3 +106,43 @@ def test_unbuilt_direct_variant_is_rejected(monkeypatch):
         with pytest.raises(F.FdtdError) as e:
             F.Sim(make(F, "vacuum", precision=F.FDTD_FP32))
         assert e.value.status == 1 and "not built" in str(e.value)
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+@pytest.mark.parametrize("name,count", [("sphere_au", 1), ("sphere_big", 3), ("hydro", 2), ("slab", 5)])
+def test_batch_blocks_agree_with_single_runs(name, count, prec):
+    """Batches under and over the tuner's size, members whose planes do not
+    fill a block's groups, one member at oblique incidence (its TFSF launch
+    runs beside the others' passes) and, after the batch, a member stepped by
+    itself."""
+    params = [make(F, name, precision=prec, NCELLZ=make(F, name).NCELLZ + i) for i in range(count)]
+    if count > 2:
+        params[1].update(inc_theta_deg=20.0, inc_phi_deg=15.0)
+    b = F.Batch(params)
+    b.step(133)
+    for i, p in enumerate(params):
+        alone = F.Sim(p)
+        alone.step(140)
+        b.sim(i).step(7)
+        for c in range(6):
+            np.testing.assert_array_equal(b.sim(i).field(c), alone.field(c), err_msg=f"member {i} component {c}")
+        np.testing.assert_array_equal(b.sim(i).spectra(), alone.spectra())
+        alone.close()
+    b.close()
+
+
+def test_batch_with_the_staged_passes(monkeypatch):
+    """A batch whose members the direct passes do not take."""
+    monkeypatch.setenv("FDTD_PASS", "staged:4:1:16:4")
+    params = [make(F, n, precision=F.FDTD_FP32) for n in ("sphere_au", "sphere_big")]
+    b = F.Batch(params)
+    b.step(140)
+    monkeypatch.delenv("FDTD_PASS")
+    for i, p in enumerate(params):
+        alone = F.Sim(p)
+        alone.step(140)
+        for c in range(6):
+            np.testing.assert_array_equal(b.sim(i).field(c), alone.field(c), err_msg=f"member {i} component {c}")
+        np.testing.assert_array_equal(b.spectra(i), alone.spectra())
+        alone.close()
+    b.close()
