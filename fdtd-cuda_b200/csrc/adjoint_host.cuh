@@ -61,12 +61,8 @@ struct fdtd_sim::Adjoint {
   int rec_off[3] = {0, 0, 0};
   double* grho[3] = {nullptr, nullptr, nullptr};
   double* gpar = nullptr;
+  int ngpar = 0;  // blocks with a share in it
   int* step = nullptr;
-  // gather tables per gather (0 = H, 1 = E): the staged tiles and the
-  // one-plane blocks of the other tiles, which the fused gathers take
-  std::unique_ptr<DevBuf> gtab[2][2];
-  int ngt[2][2] = {{0, 0}, {0, 0}};
-  bool tabs = false;
   // graphs of one full segment: the recompute (DFT off, recording on) and
   // the reverse sweep; replayed for every full segment
   cudaGraphExec_t g_rec = nullptr, g_adj = nullptr;
@@ -443,6 +439,12 @@ static fdtd_status adj_prepare(fdtd_sim* s) {
       CUDA_TRY(A.alloc(&a.lpE_F[c][slot], ce, true));
       CUDA_TRY(A.alloc(&a.lpH_N[c][slot], ch, true));
       CUDA_TRY(A.alloc(&a.lpH_F[c][slot], ch, true));
+      // the direct form's: near and far together, two buffers
+      const size_t row = (size_t)s->NZ * s->NY * view<T>(s).cp[0].W;
+      a.fEn[c][slot] = ax == 0 ? row : 2 * ce;
+      a.fHn[c][slot] = ax == 0 ? row : 2 * ch;
+      CUDA_TRY(A.alloc(&a.fE[c][slot], 2 * a.fEn[c][slot], true));
+      CUDA_TRY(A.alloc(&a.fH[c][slot], 2 * a.fHn[c][slot], true));
     }
   long long slots = 0;
   for (int c = 0; c < 3; c++) {
@@ -466,10 +468,10 @@ static fdtd_status adj_prepare(fdtd_sim* s) {
         CUDA_TRY(A.alloc(&a.lN[c][r], std::max(1, s->nmetal[c]), true));
       }
   }
-  CUDA_TRY(A.alloc(&a.gpar, 2, true));
+  A.ngpar = (int)std::max(1LL, (slots + 127) / 128);
+  CUDA_TRY(A.alloc(&a.gpar, 2 * (size_t)A.ngpar, true));
   A.gpar = a.gpar;
-  CUDA_TRY(A.alloc(&a.step, 1, false));
-  CUDA_TRY(A.alloc(&a.flags, s->ncell, false));
+  CUDA_TRY(A.alloc(&a.step, 2, false));
   A.step = a.step;
   A.rec_slots = std::max(1LL, slots);  // the record itself: adj_record_alloc
   // derivatives of the metal's coupling and dynamics coefficients with
@@ -518,98 +520,15 @@ static fdtd_status adj_sweep(fdtd_sim* s) {
   const int nsel = (int)A.sel.size();
   const double* fsel = static_cast<const double*>(A.fsel->p) + (size_t)nsel * 12;
   const int total = A.tend + 1;
-  // fused gathers (the default; FDTD_ADJ_FUSED=0 selects the coefficient
-  // arrays everywhere) need chh == 1
+  // the direct form (the default; FDTD_ADJ_FUSED=0 selects the coefficient
+  // arrays) needs chh = cee = 1 and 32-bit cell offsets
   const char* fenv = std::getenv("FDTD_ADJ_FUSED");
-  bool fused = s->su.Chh == 1.0 && !(fenv && fenv[0] == '0');
-  SlabShell she, shh;
-  {
-    const int n3[3] = {s->NX, s->NY, s->NZ};
-    int lo_e[3], lo_h[3], hi[3];
-    for (int ax = 0; ax < 3; ax++) {
-      lo_e[ax] = s->su.Nc[ax] + 1;
-      lo_h[ax] = s->su.Nc[ax];
-      hi[ax] = s->su.F[ax];
-    }
-    she.init(n3, lo_e, hi);
-    shh.init(n3, lo_h, hi);
-    if (she.total() >= (1LL << 32) || shh.total() >= (1LL << 32)) fused = false;  // 32-bit shell indices
-  }
-  const dim3 gtile((unsigned)((s->NX + 31) / 32), (unsigned)((s->NY + 7) / 8), (unsigned)s->NZ);
-  if (fused) adj_build_flags<T><<<gtile, dim3(32, 8)>>>(view<T>(s), a.flags);
-  // staged tiles: 32 x kAdjTY x kAdjKC boxes whose cells and halo (+1 for
-  // the H gather, -1 for the E gather) lie away from the CPML slabs, the
-  // grid's faces and the material box; the other tiles go to the fused
-  // gathers, one plane per block.  A tile keeps a CTA on 16 planes: on a
-  // small grid too few of them would run (fewer than 4 a multiprocessor),
-  // and the fused gathers win there; FDTD_ADJ_STAGED=1 / 0 forces either.
-  const char* senv = std::getenv("FDTD_ADJ_STAGED");
-  int nsm = 148;
-  CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
-  const long long ntiles =
-      (long long)((s->NX + 31) / 32) * ((s->NY + 7) / 8) * ((s->NZ + kAdjKC - 1) / kAdjKC);
-  const bool staged = fused && (senv ? senv[0] != '0' : ntiles >= 4LL * nsm);
-  if (staged && !A.tabs) {
-    static_assert(kAdjTY == 8, "the staged tiles and the fused gathers' blocks share the 32 x 8 xy grid");
-    const int nbx = (s->NX + 31) / 32, nby = (s->NY + 7) / 8, nbz = (s->NZ + kAdjKC - 1) / kAdjKC;
-    for (int g = 0; g < 2; g++) {
-      const int lo_off = g == 0 ? 0 : -1, hi_off = g == 0 ? 1 : 0;
-      std::vector<int4> v[2];
-      for (int bz = 0; bz < nbz; bz++)
-        for (int by = 0; by < nby; by++)
-          for (int bx = 0; bx < nbx; bx++) {
-            const int lo[3] = {bx * 32 + lo_off, by * 8 + lo_off, bz * kAdjKC + lo_off};
-            const int hi[3] = {bx * 32 + 31 + hi_off, by * 8 + 7 + hi_off,
-                               std::min(s->NZ, (bz + 1) * kAdjKC) - 1 + hi_off};
-            bool inside = true, off_mat = false;
-            for (int ax = 0; ax < 3; ax++) {
-              inside = inside && lo[ax] >= s->su.Nc[ax] + 1 && hi[ax] < s->su.F[ax];
-              off_mat = off_mat || hi[ax] < s->mat_lo[ax] || lo[ax] >= s->mat_hi[ax];
-            }
-            if (inside && off_mat) {
-              v[0].push_back(make_int4(bx, by, bz, 0));
-            } else {
-              for (int k = bz * kAdjKC; k < std::min(s->NZ, (bz + 1) * kAdjKC); k++) v[1].push_back(make_int4(bx, by, k, 0));
-            }
-          }
-      for (int q = 0; q < 2; q++) {
-        auto b = std::make_unique<DevBuf>();
-        CUDA_TRY(b->alloc(std::max<size_t>(1, v[q].size()) * sizeof(int4)));
-        if (!v[q].empty()) CUDA_TRY(cudaMemcpy(b->p, v[q].data(), v[q].size() * sizeof(int4), cudaMemcpyHostToDevice));
-        A.gtab[g][q] = std::move(b);
-        A.ngt[g][q] = (int)v[q].size();
-      }
-    }
-    const int smem = (int)(kAdjS * StageLayout<T, kAdjTY>::STAGE * sizeof(T));
-    CUDA_TRY(cudaFuncSetAttribute(adj_gather_h_staged<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CUDA_TRY(cudaFuncSetAttribute(adj_gather_e_staged<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    A.tabs = true;
-  }
-  const size_t gsmem = kAdjS * StageLayout<T, kAdjTY>::STAGE * sizeof(T);
-  // one gather: the staged tiles and the fused blocks (disjoint outputs,
-  // inputs they do not write); returns the launches
-  auto gather = [&](int g, cudaStream_t stream) -> int {
-    if (!staged) {
-      if (g == 0) adj_gather_h_fused<T><<<gtile, dim3(32, 8), 0, stream>>>(view<T>(s), a, nullptr);
-      else adj_gather_e_fused<T><<<gtile, dim3(32, 8), 0, stream>>>(view<T>(s), a, nullptr);
-      return 1;
-    }
-    int k = 0;
-    const int4* tt = static_cast<const int4*>(A.gtab[g][0]->p);
-    const int4* lt = static_cast<const int4*>(A.gtab[g][1]->p);
-    const int* n = A.ngt[g];
-    if (n[1]) {
-      if (g == 0) adj_gather_h_fused<T><<<n[1], dim3(32, 8), 0, stream>>>(view<T>(s), a, lt);
-      else adj_gather_e_fused<T><<<n[1], dim3(32, 8), 0, stream>>>(view<T>(s), a, lt);
-      k++;
-    }
-    if (n[0]) {
-      if (g == 0) adj_gather_h_staged<T><<<n[0], dim3(32, kAdjTY), gsmem, stream>>>(view<T>(s), a, tt);
-      else adj_gather_e_staged<T><<<n[0], dim3(32, kAdjTY), gsmem, stream>>>(view<T>(s), a, tt);
-      k++;
-    }
-    return k;
-  };
+  const bool direct = s->su.Chh == 1.0 && s->su.Cee == 1.0 && s->ncell < ((size_t)1 << 31) && !(fenv && fenv[0] == '0');
+  // planes per thread: as the forward's E pass, whose loads these are, but
+  // short runs (the neighbour plane's coefficients are computed once a run)
+  const int kz = std::min(std::max(s->ecfg.kz, 2), 8);
+  const unsigned nbx = (unsigned)((s->plane / Vec<T>::N + kFlatThreads - 1) / kFlatThreads);
+  const unsigned gz = nbx * (unsigned)((s->NZ + kz - 1) / kz);
   // the dispersive cells' transposed update: the local model in one
   // launch; the hydrodynamic model as its three phases in reverse order,
   // then the current update
@@ -631,16 +550,11 @@ static fdtd_status adj_sweep(fdtd_sim* s) {
       adj_source<T><<<dim3((maxn + 255) / 256, 12), 256, 0, stream>>>(view<T>(s), s->dft, a,
                                                                        static_cast<const double2*>(A.P->p), fsel,
                                                                        nsel, s->dft.rows, A.face_mask);
-    if (fused) {
-      if (she.total() > 0)
-        adj_e_slab<T><<<(unsigned)((she.total() + 255) / 256), 256, 0, stream>>>(view<T>(s), a, she);
+    if (direct) {
       const int kd = ntot > 0 ? launch_design(stream) : 0;
-      const int kg = gather(0, stream);
-      if (shh.total() > 0)
-        adj_h_slab<T><<<(unsigned)((shh.total() + 255) / 256), 256, 0, stream>>>(view<T>(s), a, shh);
-      const int kg2 = gather(1, stream);
-      adj_step_back<<<1, 1, 0, stream>>>(A.step);
-      return 1 + kg + kg2 + (she.total() > 0) + (shh.total() > 0) + kd + (n % every_dft == 0);
+      adj_h_flat<T><<<gz, kFlatThreads, 0, stream>>>(view<T>(s), a, nbx, kz);
+      adj_e_flat<T><<<gz, kFlatThreads, 0, stream>>>(view<T>(s), a, nbx, kz);  // moves the adjoint clock
+      return 2 + kd + (n % every_dft == 0);
     }
     adj_e_coef<T><<<gc, 256, 0, stream>>>(view<T>(s), a);
     const int kd = ntot > 0 ? launch_design(stream) : 0;
@@ -742,7 +656,13 @@ static fdtd_status adj_backward(fdtd_sim* s, float* dL_drho, size_t count, doubl
       dL_drho[q] = (float)v;
     }
   }
-  if (dL_dparams) CUDA_TRY(cudaMemcpy(dL_dparams, A.gpar, 2 * sizeof(double), cudaMemcpyDeviceToHost));
+  if (dL_dparams) {
+    std::vector<double> g(2 * (size_t)A.ngpar);
+    CUDA_TRY(cudaMemcpy(g.data(), A.gpar, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    dL_dparams[0] = dL_dparams[1] = 0.0;
+    for (int b = 0; b < A.ngpar; b++)
+      for (int p = 0; p < 2; p++) dL_dparams[p] += g[2 * (size_t)b + p];
+  }
   return FDTD_OK;
 }
 

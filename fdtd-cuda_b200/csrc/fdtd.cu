@@ -20,6 +20,7 @@
 #include "flat.cuh"
 #include "boundary.cuh"
 #include "adjoint.cuh"
+#include "adj_flat.cuh"
 #include "snapshot.cuh"
 #include "setup.h"
 

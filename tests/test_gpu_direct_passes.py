@@ -146,3 +146,29 @@ def test_batch_with_the_staged_passes(monkeypatch):
         np.testing.assert_array_equal(b.spectra(i), alone.spectra())
         alone.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+@pytest.mark.parametrize("nx,ny,nonlocal_", [(0, 0, 0), (1, 3, 0), (2, 1, 3), (3, 2, 0), (5, 0, 3)])
+def test_direct_adjoint_agrees_with_coefficient_arrays(nx, ny, nonlocal_, prec, monkeypatch):
+    """Row lengths of every remainder and rows that end inside a warp, both
+    dispersive models, a dielectric slab under the design box's metal: the
+    same sums in the same order; the source's atomics at the corners shared
+    by two flux faces leave rounding."""
+    gold = dict(metal_custom=1, eps_inf=1.1431, omega_D=1.3202e16, gamma_D=1.0805e14, cp_A=(0.26698, 3.0834),
+                cp_phi=(-1.2371, -1.0968), cp_Omega=(3.8711e15, 4.1684e15), cp_Gamma=(4.4642e14, 2.3555e15))
+    out = []
+    for mode in ("1", "0"):
+        monkeypatch.setenv("FDTD_ADJ_FUSED", mode)
+        s = F.Sim(make(F, "disks_slab", precision=prec, NCELLX=27 + nx, NCELLY=25 + ny, Tend=260, NONLOCAL=nonlocal_,
+                       disk_diameter=4e-9, disk_nx=1, disk_ny=1, slab_thickness=4e-9,
+                       design_box=[18, 22, 17, 20, 16, 19], **gold))
+        s.set_design(np.random.default_rng(4).uniform(0, 1, (3, 3, 4)).astype(np.float32))
+        value = s.forward([2, 5], 60)
+        out.append((value, *s.backward()))
+        s.close()
+    assert out[0][0] == out[1][0]
+    tol = 1e-11 if prec == F.FDTD_FP64 else 1e-5
+    assert np.abs(out[1][1]).max() > 0
+    assert np.abs(out[0][1] - out[1][1]).max() <= tol * np.abs(out[1][1]).max()
+    np.testing.assert_allclose(out[0][2], out[1][2], rtol=tol)
