@@ -559,6 +559,8 @@ __global__ void adj_gather_e(const __grid_constant__ SimView<T> s, const __grid_
   a.lE[2][id] += (py ? a.a[0][0][id - sy] : T(0)) - a.a[0][0][id] + (px ? a.a[1][1][id - sx] : T(0)) - a.a[1][1][id];
 }
 
+constexpr int kAdjPhasors = 64;  // per round of adj_source
+
 // Objective derivative at a DFT sample step n: for every flux-face cell and
 // tangential component of the faces in face_mask (bit b*6+f: box b, face
 // f), g = sum_m Re(P_m conj(w_m)) with w_m = exp(i 2 pi (n + delta) dt f_m)
@@ -573,8 +575,35 @@ __global__ void adj_source(const __grid_constant__ SimView<T> s, const __grid_co
   const DftFace F = d.face[f];
   const int nc = F.na * F.nb;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nc) return;
   const int n = *a.step;
+  // the phasors are the same for every cell: once per block, kAdjPhasors
+  // frequencies at a time
+  __shared__ double2 w[2][kAdjPhasors];
+  auto phasors = [&](int m0) {
+    __syncthreads();
+    if (threadIdx.x < 2 * kAdjPhasors) {
+      const int h = threadIdx.x / kAdjPhasors, m = threadIdx.x - h * kAdjPhasors;
+      if (m0 + m < nsel) {
+        const double ph = (double)(float)2.0 * 3.1415926535897932384626433832795 * (n + (h ? 0.5 : 1.0)) * d.dt * fsel[m0 + m];
+        double sv, cv;
+        sincos(ph, &sv, &cv);
+        w[h][m] = make_double2(cv, sv);
+      }
+    }
+    __syncthreads();
+  };
+  double g[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int m0 = 0; m0 < nsel; m0 += kAdjPhasors) {
+    phasors(m0);
+    if (q >= nc) continue;
+    for (int m = m0; m < min(nsel, m0 + kAdjPhasors); m++)
+#pragma unroll
+      for (int cs = 0; cs < 4; cs++) {
+        const double2 p = P[(size_t)m * prows + F.row0 + (long long)cs * F.npad + q], v = w[cs < 2 ? 0 : 1][m - m0];
+        g[cs] += p.x * v.x + p.y * v.y;
+      }
+  }
+  if (q >= nc) return;
   const int u = q / F.nb, v = q - u * F.nb;
   int ijk[3];
   const int a1 = F.ax == 0 ? 1 : 0, a2 = F.ax == 2 ? 1 : 2;
@@ -584,19 +613,9 @@ __global__ void adj_source(const __grid_constant__ SimView<T> s, const __grid_co
   const size_t id = fidx(s.PX, s.plane, ijk[0], ijk[1], ijk[2]);
 #pragma unroll
   for (int cs = 0; cs < 4; cs++) {
-    const long long row = F.row0 + (long long)cs * F.npad + q;
-    const double del = cs < 2 ? 1.0 : 0.5;
-    double g = 0.0;
-    for (int m = 0; m < nsel; m++) {
-      const double ph = (double)(float)2.0 * 3.1415926535897932384626433832795 * (n + del) * d.dt * fsel[m];
-      double sv, cv;
-      sincos(ph, &sv, &cv);
-      const double2 p = P[(size_t)m * prows + row];
-      g += p.x * cv + p.y * sv;
-    }
     const int comp = F.comp[cs];
     T* dst = comp < 3 ? a.lE[comp] : a.lH[comp - 3];
-    atomicAdd(dst + id, (T)g);
+    atomicAdd(dst + id, (T)g[cs]);
   }
 }
 
