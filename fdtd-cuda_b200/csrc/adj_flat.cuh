@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
   const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
   const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
   const unsigned PXV = (unsigned)PX / N, NV = PXV * (unsigned)NY, plane = (unsigned)s.plane;
-  unsigned vq = xb * kFlatThreads + threadIdx.x;
+  unsigned vq = xb * blockDim.x + threadIdx.x;
   const bool in = vq < NV;
   if (!in) vq = NV - 1;
   const int j = (int)(vq / PXV), i0 = (int)(vq - (unsigned)j * PXV) * N;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
   const unsigned kb = blockIdx.x / nbx, xb = blockIdx.x - kb * nbx;
   const int NX = s.NX, NY = s.NY, NZ = s.NZ, PX = s.PX;
   const unsigned PXV = (unsigned)PX / N, NV = PXV * (unsigned)NY, plane = (unsigned)s.plane;
-  unsigned vq = xb * kFlatThreads + threadIdx.x;
+  unsigned vq = xb * blockDim.x + threadIdx.x;
   const bool in = vq < NV;
   if (!in) vq = NV - 1;
   const int j = (int)(vq / PXV), i0 = (int)(vq - (unsigned)j * PXV) * N;

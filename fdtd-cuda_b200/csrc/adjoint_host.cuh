@@ -527,7 +527,8 @@ static fdtd_status adj_sweep(fdtd_sim* s) {
   // planes per thread: as the forward's E pass, whose loads these are, but
   // short runs (the neighbour plane's coefficients are computed once a run)
   const int kz = std::min(std::max(s->ecfg.kz, 2), 8);
-  const unsigned nbx = (unsigned)((s->plane / Vec<T>::N + kFlatThreads - 1) / kFlatThreads);
+  const int thr = s->ecfg.ring ? kFlatThreads : s->ecfg.thr;
+  const unsigned nbx = (unsigned)((s->plane / Vec<T>::N + thr - 1) / thr);
   const unsigned gz = nbx * (unsigned)((s->NZ + kz - 1) / kz);
   // the dispersive cells' transposed update: the local model in one
   // launch; the hydrodynamic model as its three phases in reverse order,
@@ -552,8 +553,8 @@ static fdtd_status adj_sweep(fdtd_sim* s) {
                                                                        nsel, s->dft.rows, A.face_mask);
     if (direct) {
       const int kd = ntot > 0 ? launch_design(stream) : 0;
-      adj_h_flat<T><<<gz, kFlatThreads, 0, stream>>>(view<T>(s), a, nbx, kz);
-      adj_e_flat<T><<<gz, kFlatThreads, 0, stream>>>(view<T>(s), a, nbx, kz);  // moves the adjoint clock
+      adj_h_flat<T><<<gz, thr, 0, stream>>>(view<T>(s), a, nbx, kz);
+      adj_e_flat<T><<<gz, thr, 0, stream>>>(view<T>(s), a, nbx, kz);  // moves the adjoint clock
       return 2 + kd + (n % every_dft == 0);
     }
     adj_e_coef<T><<<gc, 256, 0, stream>>>(view<T>(s), a);

@@ -82,7 +82,7 @@ struct fdtd_sim {
   struct PassCfg { int minb = 1, ty = 4, kchunk = 16, staged = 1, stages = 4, eminb = 1, estages = 4, pdl = 0, tma = 0, etma = 0; float ms = 0;
     // direct pass (flat.cuh): planes per thread, and whether they are copied
     // ahead into shared memory; kz = 0 = the staged pass
-    int kz = 0, ring = 0; };
+    int kz = 0, ring = 0, thr = kFlatThreads; };
   // pass tiles for one (tile height, z-chunk): the interior box of tiles
   // that touch no CPML slab and the table of the others
   struct TileSet {
@@ -1166,12 +1166,13 @@ static void launch_ex(bool pdl, void (*kern)(P...), dim3 g, dim3 blk, size_t sme
 // cells' share of it (the hydrodynamic currents in the H launch, the E updates
 // in the E launch).
 template <typename T, bool EPASS>
-static void launch_flat(fdtd_sim* s, int kz, int ring, cudaStream_t st, bool line = false, bool cells = false) {
+static void launch_flat(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st, bool line = false, bool cells = false) {
+  const int kz = c.kz, ring = c.ring, thr = ring ? kFlatThreads : c.thr;
   const unsigned nv = (unsigned)(s->plane / Vec<T>::N), ntot = (unsigned)(s->nmetal[0] + s->nmetal[1] + s->nmetal[2]);
   const bool hydro = s->su.hydro != 0;
-  FlatGrid g{(nv + kFlatThreads - 1) / kFlatThreads, 0, kz, line ? 1 : 0};
-  if (cells && (EPASS || hydro)) g.nrole = (ntot + kFlatThreads - 1) / kFlatThreads;
-  const dim3 grid(g.nbx * (unsigned)((s->NZ + kz - 1) / kz) + g.nrole + g.line), blk(kFlatThreads);
+  FlatGrid g{(nv + thr - 1) / thr, 0, kz, line ? 1 : 0};
+  if (cells && (EPASS || hydro)) g.nrole = (ntot + thr - 1) / thr;
+  const dim3 grid(g.nbx * (unsigned)((s->NZ + kz - 1) / kz) + g.nrole + g.line), blk(thr);
   const SimView<T>& v = view<T>(s);
   const MetalView<T>& m = mview<T>(s);
   const size_t smem = ring ? kFlatRingBytes : 0;
@@ -1220,7 +1221,7 @@ static cudaError_t flat_attributes() {
 template <typename T, bool EPASS>
 static int launch_pass_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st, bool chained = false) {
   if (c.kz) {
-    launch_flat<T, EPASS>(s, c.kz, c.ring, st);
+    launch_flat<T, EPASS>(s, c, st);
     return 1;
   }
   const fdtd_sim::TileSet& ts = tiles(s, c);
@@ -1278,7 +1279,7 @@ static int launch_e_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st
 // between: timed on the zero state like the staged shapes.  Untimed (FDTD_TUNE=0,
 // batch members, under 2^18 cells) the most planes, up to 8, that leave two
 // blocks a multiprocessor, copied ahead from 4 planes on.
-// FDTD_PASS=flat:KZ[:RING] fixes them.
+// FDTD_PASS=flat:KZ[:RING[:THREADS]] fixes them.
 template <typename T>
 static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force) {
   if (s->fused_tfsf) CUDA_TRY((flat_attributes<T, true>()));
@@ -1293,12 +1294,14 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
   while (def.kz < 8 && nbx * ((s->NZ + 2 * def.kz - 1) / (2 * def.kz)) >= 2 * sms) def.kz *= 2;
   def.ring = def.kz >= 4;
   if (force) {
-    if (std::sscanf(force, "flat:%d:%d", &def.kz, &def.ring) < 1 || def.kz < 1 || def.ring < 0 || def.ring > 1)
+    if (std::sscanf(force, "flat:%d:%d:%d", &def.kz, &def.ring, &def.thr) < 1 || def.kz < 1 || def.ring < 0 ||
+        def.ring > 1 || (def.thr != 128 && def.thr != kFlatThreads))
       return fail(FDTD_ERR_INVALID, "FDTD_PASS names a pass variant that is not built");
   }
   auto report = [](fdtd_sim::PassCfg& c) {
     c.kchunk = c.kz;
     c.stages = c.estages = c.ring ? kFlatRing : 1;
+    c.minb = c.eminb = 2 * kFlatThreads / (c.ring ? kFlatThreads : c.thr);
   };
   report(def);
   s->hcfg = s->ecfg = def;
@@ -1332,19 +1335,21 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
     float best_ms = 1e30f;
     for (int kz : kzs) {
       if (kz > s->NZ) continue;
-      for (int ring = 0; ring < 2; ring++) {
-        if (ring ? !big || kz < 4 : big && (kz == 6 || kz == 12 || kz > 16)) continue;
+      for (int form = 0; form < 3; form++) {  // 256 threads, 128 threads, ring
+        const int ring = form == 2;
+        if (ring ? !big || kz < 4 : big && (form == 1 || kz == 6 || kz == 12 || kz > 16)) continue;
         fdtd_sim::PassCfg c = def;
         c.kz = kz;
         c.ring = ring;
+        c.thr = form == 1 ? 128 : kFlatThreads;
         report(c);
         cudaGraph_t g = nullptr;
         cudaGraphExec_t x = nullptr;
         err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
         for (int r = 0; r < reps; r++) {
-          if (pass == 0) launch_flat<T, false>(s, kz, ring, st);
-          else launch_flat<T, true>(s, kz, ring, st);
+          if (pass == 0) launch_flat<T, false>(s, c, st);
+          else launch_flat<T, true>(s, c, st);
         }
         err = cudaStreamEndCapture(st, &g);
         if (err == cudaSuccess) err = cudaGraphInstantiate(&x, g, 0);
@@ -1361,8 +1366,8 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
         if (err != cudaSuccess) break;
         c.ms = ms / reps;
         if (verbose)
-          std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread%s: %.4f ms\n", pass == 0 ? "H" : "E", kz,
-                       ring ? ", copied ahead" : "", c.ms);
+          std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread, %d threads%s: %.4f ms\n", pass == 0 ? "H" : "E",
+                       kz, c.thr, ring ? ", copied ahead" : "", c.ms);
         if (c.ms < best_ms) {
           best_ms = c.ms;
           best = c;
@@ -1573,7 +1578,7 @@ static void launch_e(fdtd_sim* s, cudaStream_t st) {
       hydro_p<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
       s->kernels++;
     }
-    launch_flat<T, true>(s, s->ecfg.kz, s->ecfg.ring, st, false, true);
+    launch_flat<T, true>(s, s->ecfg, st, false, true);
     s->kernels++;
     return;
   }
@@ -1714,9 +1719,9 @@ static void enqueue_step(fdtd_sim* s, cudaStream_t st) {
     // launch's blocks, resident early, take the slots that free first and the
     // single-wave passes end up unevenly spread (97 x 89 x 93 FP64 33.0 us a step
     // against 26.5, 96^3 20.8 against 18.3, 256^3 FP32 250.3 against 246.2).
-    launch_flat<T, false>(s, s->hcfg.kz, s->hcfg.ring, st, true, true);
+    launch_flat<T, false>(s, s->hcfg, st, true, true);
     launch_tfsf<T>(s, st);
-    launch_flat<T, true>(s, s->ecfg.kz, s->ecfg.ring, st, false, true);
+    launch_flat<T, true>(s, s->ecfg, st, false, true);
     s->kernels += 2;
     if (s->line.dft_every > 0 && s->t % s->line.dft_every == 0) sample_and_contract<T>(s, st);
     if (s->snap_on) launch_snap<T>(s, st);

@@ -50,6 +50,8 @@ __device__ __forceinline__ Vec<T> zerov() {
   return r;
 }
 
+// Threads per block of the forms with a ring, and the most the others take: those
+// also run with 128, which fills the last wave of a small grid better.
 constexpr int kFlatThreads = 256;
 
 // A thread's own vectors of the planes to come, copied into shared memory
@@ -375,13 +377,13 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
   }
   if (HYDRO) {
     if (b < g.nrole) {
-      hydro_p_any(s, m, s.clk->th, (int)(b * kFlatThreads + threadIdx.x));
+      hydro_p_any(s, m, s.clk->th, (int)(b * blockDim.x + threadIdx.x));
       return;
     }
     b -= g.nrole;
   }
   const unsigned kb = b / g.nbx, xb = b - kb * g.nbx;
-  h_flat_cells<T, RING, TFSF>(s, xb * kFlatThreads + threadIdx.x, (int)kb * g.kz, g.kz);
+  h_flat_cells<T, RING, TFSF>(s, xb * blockDim.x + threadIdx.x, (int)kb * g.kz, g.kz);
 }
 
 // E pass (UPDATE_ex/ey/ez, main.cu:1048-1912) of the vector vq, planes k0 ..
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
   if (b == 0 && threadIdx.x == 0) s.clk->th = s.clk->t;
   if (KIND) {
     if (b < g.nrole) {
-      const int q = (int)(b * kFlatThreads + threadIdx.x), t = s.clk->t - 1;
+      const int q = (int)(b * blockDim.x + threadIdx.x), t = s.clk->t - 1;
       if (KIND == 1) metal_e_cell(s, m, t, q);
       else hydro_e_any(s, m, t, q);
       return;
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
     b -= g.nrole;
   }
   const unsigned kb = b / g.nbx, xb = b - kb * g.nbx;
-  e_flat_cells<T, RING, TFSF>(s, xb * kFlatThreads + threadIdx.x, (int)kb * g.kz, g.kz);
+  e_flat_cells<T, RING, TFSF>(s, xb * blockDim.x + threadIdx.x, (int)kb * g.kz, g.kz);
 }
 
 }  // namespace fdtd

@@ -15,7 +15,7 @@ from cases import make
 
 pytestmark = pytest.mark.gpu
 
-SPECS = ("flat:1", "flat:5", "flat:2:1", "flat:8:1", "flat:64:1", "flat:200")
+SPECS = ("flat:1", "flat:5", "flat:3:0:128", "flat:2:1", "flat:8:1", "flat:64:1", "flat:200")
 
 
 def fields(name, prec, spec, monkeypatch, steps, **over):
@@ -82,7 +82,7 @@ def test_split_entry_points_agree_with_the_fused_step(name, tfsf, monkeypatch):
 @pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
 @pytest.mark.parametrize("dx", range(8))
 def test_every_row_remainder(dx, prec, monkeypatch):
-    agree("sphere_au", prec, ("flat:1", "flat:7:1"), monkeypatch, steps=90, NCELLX=21 + dx, NCELLY=22 - dx % 3)
+    agree("sphere_au", prec, ("flat:1", "flat:7:1", "flat:2:0:128"), monkeypatch, steps=90, NCELLX=21 + dx, NCELLY=22 - dx % 3)
 
 
 def test_tuned_and_untuned_direct_passes_agree(monkeypatch):
@@ -101,7 +101,7 @@ def test_tuned_and_untuned_direct_passes_agree(monkeypatch):
 
 
 def test_unbuilt_direct_variant_is_rejected(monkeypatch):
-    for spec in ("flat:0", "flat:4:2"):
+    for spec in ("flat:0", "flat:4:2", "flat:4:0:96"):
         monkeypatch.setenv("FDTD_PASS", spec)
         with pytest.raises(F.FdtdError) as e:
             F.Sim(make(F, "vacuum", precision=F.FDTD_FP32))
