@@ -1333,11 +1333,18 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
   for (int pass = 0; pass < 2 && err == cudaSuccess; pass++) {
     fdtd_sim::PassCfg& best = pass == 0 ? s->hcfg : s->ecfg;
     float best_ms = 1e30f;
-    for (int kz : kzs) {
-      if (kz > s->NZ) continue;
-      for (int form = 0; form < 3; form++) {  // 256 threads, 128 threads, ring
-        const int ring = form == 2;
+    int best_kz = 0;  // of the blocks of 256 threads
+    bool past = false;
+    for (int form = 0; form < 3; form++) {  // 256 threads, 128 threads, ring
+      for (size_t q = 0; q < kzs.size() && err == cudaSuccess; q++) {
+        const int kz = kzs[q], ring = form == 2;
+        if (kz > s->NZ) continue;
         if (ring ? !big || kz < 4 : big && (form == 1 || kz == 6 || kz == 12 || kz > 16)) continue;
+        // a small grid is created in a few milliseconds: no longer runs of planes
+        // once they lose by a third, and 128 threads only next to the best 256
+        if (form == 0 && !big && past) continue;
+        if (form == 1 && kz != best_kz && (q == 0 || kzs[q - 1] != best_kz) && (q + 1 >= kzs.size() || kzs[q + 1] != best_kz))
+          continue;
         fdtd_sim::PassCfg c = def;
         c.kz = kz;
         c.ring = ring;
@@ -1368,9 +1375,11 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
         if (verbose)
           std::fprintf(stderr, "[fdtd tune] %s pass, %d planes a thread, %d threads%s: %.4f ms\n", pass == 0 ? "H" : "E",
                        kz, c.thr, ring ? ", copied ahead" : "", c.ms);
+        past = past || c.ms > 1.33f * best_ms;
         if (c.ms < best_ms) {
           best_ms = c.ms;
           best = c;
+          if (form == 0) best_kz = kz;
         }
       }
     }
