@@ -269,7 +269,7 @@ def batch_members(mod, n=64, steps=3000, seed=BATCH_SEED):
 
 def batch_bench(mod, torch, stream, sp, dev, n, steps):
     """sims/s of the batched path (fdtd_batch_run: all members in one
-    persistent pass kernel per half step) against the same members run one
+    launch per half step) against the same members run one
     after another with fdtd_run, both timed with CUDA events on one stream;
     creation is outside both timed regions."""
     params = batch_members(mod, n, steps)
@@ -686,7 +686,7 @@ def main():
     sb = step_bytes(d, p32, tune, 4)
     step_ms = ms / args.steps / BLOCK
     step_gbs = sb["total"] / (step_ms / 1e3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "e_pass_s<float> (Yee + CPML E pass, whole grid)",
+    roofline = {"bound": "hbm", "kernel": "e_flat<float> (Yee + CPML E pass, whole grid)",
                 "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4),
                 "traffic": profile_traffic("e_pass_fp32_256"),

@@ -18,7 +18,11 @@
 //
 // What this replaced: slab kernels that wrote coefficient arrays for the CPML
 // cells, and gathers that read flags and arrays for every cell (19 to 24 values
-// a cell and sub-step there against 9).
+// a cell and sub-step there against 9).  Backward, us a step: FP32 96^3 56.5 to
+// 25.9, 65x71x61 36.8 to 22.4, 184x168x129 hydrodynamic 263 to 167; FP64 160^3
+// 331 to 211.  Bound by latency up to 128^3, above it by DRAM with 16 warps a
+// multiprocessor; the copy-ahead ring of flat.cuh gave nothing here (168 to 169),
+// nor did the transposed current update as blocks of adj_h_flat (167 to 166).
 #pragma once
 #include "adjoint.cuh"
 #include "flat.cuh"

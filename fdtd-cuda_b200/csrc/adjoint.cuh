@@ -6,8 +6,9 @@
 //
 //   lambda^n = M^T lambda^{n+1} + dL/dx^n,   dL/drho = sum_n lambda^{n+1} (dM/drho) x^n
 //
-// The transposed Yee/CPML sub-steps are written in gather form: a first
-// kernel turns each updated component's adjoint into the coefficients of
+// The transposed Yee/CPML sub-steps are written in gather form and run as the
+// direct passes of adj_flat.cuh; the form they must agree with (and the one for
+// grids beyond 32-bit offsets) stands here: a first kernel turns each updated component's adjoint into the coefficients of
 // the field differences it read ("a" arrays, one per component and
 // difference axis) and applies the psi recursions transposed; a second
 // kernel gathers those coefficients into the adjoint of the other field
@@ -229,7 +230,7 @@ __global__ void adj_e_design(const __grid_constant__ SimView<T> s, const __grid_
 
 // ---------------------------------------------------------------------
 // Hydrodynamic cells, transposed.  The forward step (kernels.cuh) is three
-// phases: hydro_p_ex computes J^{n+1} of every cell from J^n, J^{n-1},
+// phases: hydro_p_any computes J^{n+1} of every cell from J^n, J^{n-1},
 // E^n, E^{n-1} and the pressure term over the neighbour slots' J^n and
 // N^n, then the x cells' continuity and E update; hydro_e<1> and <2> do the
 // y and z cells, whose continuity reads the x (and y) neighbours' new J and

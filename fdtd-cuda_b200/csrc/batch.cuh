@@ -15,7 +15,11 @@
 //                     every 32 samples; it contracts each member's first
 //                     ring half once that holds 64 samples
 // so the launch count per step does not grow with the member count, and
-// small members that could not fill the GPU alone share it.  Runs of
+// small members that could not fill the GPU alone share it.  A step, us, against
+// persistent staged passes over a work queue with the other kernels in launches
+// of their own: 16 members of 48-128 381 to 305, 4 of 44-60 51.7 to 22.6, 40 of
+// 48-128 875 to 700, 8 of 80-140 FP64 697 to 473; bound by DRAM for the large
+// members (16 warps a multiprocessor).  Runs of
 // 32 * dft_every steps are captured into one CUDA graph and replayed.  A batch
 // with a member that the direct passes do not take (the staged ones are forced,
 // or it is beyond their 32-bit offsets) steps its members one after another.

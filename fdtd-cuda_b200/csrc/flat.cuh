@@ -15,6 +15,20 @@
 // ring of shared-memory stages (staged.cuh) walks 8 to 32 planes per CTA
 // with a barrier each; a small grid fills the GPU only for a short chain of
 // such steps, and the CPML tiles of a large one stall on their psi loads.
+// Pass times, us, H / E, staged against this form: FP32 64^3 10.3/10.3 and
+// 6.2/6.2, 96^3 12.8/16.5 and 8.3/9.3, 128^3 24.5/23.2 and 16.1/17.1, 256^3
+// 131/141 and 120/124 (5.7 and 5.5 TB/s of algorithmic bytes), 384x384x256
+// 270/289 and 248/262; FP64 256^3 236/240 and 227/237 (6.0 and 5.8 TB/s).
+// What bounds it: up to 128^3 the latency of one thread's few planes, above it
+// DRAM, short of the copy rate because 16 warps a multiprocessor (128 registers)
+// hold the loads in flight.  Fewer registers spill (80: twice the time), psi
+// loaded after the fields costs the 256^3 E pass 124 -> 156, one plane a thread
+// everywhere re-reads planes from DRAM (H 120 -> 159), L2 prefetches of the
+// planes ahead 121 -> 130.
+//
+// The line, the dispersive cells and the TFSF increments ride in the two
+// launches: a step in seven launches on side streams was 13.5 us at 64^3 and
+// 292 us for the 256^3 dimer with these passes, in two 9.1 and 267.
 #pragma once
 #include "kernels.cuh"
 

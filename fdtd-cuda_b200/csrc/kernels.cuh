@@ -1,20 +1,24 @@
 // CUDA kernels of the FDTD time step (sm_100a).
 //
-// One time step is:
-//   h_pass      UPDATE_hx/hy/hz + H CPML (staged.cuh)
-//   tfsf_h      H half of CORRECT_X/Y/Z on the TFSF faces (boundary.cuh)
-//   line_step   UPDATE_h_inc + UPDATE_e_inc + Mur ends + source (1 CTA)
-//   tfsf_e      E half of CORRECT_X/Y/Z (boundary.cuh)
-//   e_pass      UPDATE_ex/ey/ez for non-dispersive components + E CPML
-//   metal_e / hydro_*   dispersive (Drude + 2CP, hydrodynamic) cells,
-//               compact lists
+// One time step is two launches (flat.cuh), three with the TFSF launch:
+//   h_flat      UPDATE_h_inc + UPDATE_e_inc + Mur ends + source (one block),
+//               the hydrodynamic currents (a few blocks), and
+//               UPDATE_hx/hy/hz + H CPML
+//   tfsf_apply  both halves of CORRECT_X/Y/Z on the TFSF faces (boundary.cuh):
+//               at oblique incidence and on large grids; else the passes add
+//               the increments that the line's block computed
+//   e_flat      the dispersive cells' E updates (Drude + 2CP, hydrodynamic;
+//               compact lists) and UPDATE_ex/ey/ez for the other
+//               components + E CPML
+// and beside them
 //   dft_sample  every dft_every steps: gather the flux-plane tangential
 //               components into a sample ring
 //   dft_contract once a half of the ring holds kRingSlots samples: FP64
 //               contraction of that half with the phasors into the
 //               accumulators, beside the steps that fill the other half
 // This file holds the bodies of everything but the Yee passes and the TFSF
-// tables.
+// tables.  With the staged passes (staged.cuh) the same bodies run as launches
+// of their own.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>

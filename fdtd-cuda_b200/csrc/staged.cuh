@@ -1,4 +1,5 @@
-// Shared-memory-staged E and H passes: the Yee updates of all cells with the
+// Shared-memory-staged E and H passes, the form for grids beyond the direct
+// passes' 32-bit cell offsets (flat.cuh) and for the knobs that ask for it: the Yee updates of all cells with the
 // CPML psi recursions of the six absorbing slabs fused in (UPDATE_hx/hy/hz
 // and UPDATE_ex/ey/ez with their CPML blocks; the TFSF corrections and the
 // dispersive cells are applied by the kernels of boundary.cuh and

@@ -408,7 +408,7 @@ class Sim:
 
 class Batch:
     """Independent simulations advanced together (fdtd_batch_*): the Yee
-    passes of all members share one persistent kernel per half step."""
+    passes of all members run as one launch per half step."""
 
     def __init__(self, params_list, device=0):
         self.params = list(params_list)

@@ -379,13 +379,15 @@ typedef struct fdtd_stats {
   long long kernels;
   long long steps;
   long long graph_launches;
-  /* launch shapes picked by the autotuner (min CTAs/SM, tile height,
-   * z-chunk) and their measured time per launch, for the H and E passes */
+  /* launch shapes picked by the autotuner and their measured time per launch,
+   * for the H and E passes.  Direct passes (h_staged = 0): minb CTAs/SM,
+   * kchunk planes per thread, ty unused.  Staged passes: min CTAs/SM, tile
+   * height, z-chunk */
   int h_minb, h_ty, h_kchunk, e_minb, e_ty, e_kchunk;
   float h_ms, e_ms;
   int h_staged, e_staged;  /* 1 = shared-memory pipelined pass */
-  int h_stages, e_stages;  /* its ring depth */
-  /* the same two for the launch over the CPML edge tiles */
+  int h_stages, e_stages;  /* its ring depth; direct: 4 = planes copied ahead */
+  /* the same two for the staged launch over the CPML edge tiles */
   int h_eminb, h_estages, e_eminb, e_estages;
   /* 1 = the two launches of the pass run on one stream with a programmatic
    * dependency, 0 = on two streams */
@@ -406,7 +408,7 @@ typedef struct fdtd_stats {
 } fdtd_stats;
 fdtd_status fdtd_get_stats(const fdtd_sim* s, fdtd_stats* out);
 /* Measurement hook (no counterpart in the reference): runs one Yee pass
- * (its interior-tile and CPML-edge-tile launches) reps times back to back,
+ * (its one direct launch, or its two staged ones) reps times back to back,
  * after two untimed runs, on `stream` and stores its mean device time per
  * pass, from CUDA events on that stream, in *ms.  The runs change the
  * fields: call fdtd_reset before using the simulation again. */
@@ -471,10 +473,10 @@ typedef struct fdtd_batch fdtd_batch;
  * switch, the DFT sampling period and Tend. */
 fdtd_status fdtd_batch_create(const fdtd_params* ps, int n, int device,
                               fdtd_batch** out);
-/* Advances every member by nsteps.  Per time step the two Yee passes of
- * all members run as one persistent kernel each, fed from a shared
- * (member, tile) work queue, and every other kernel of the step runs as one
- * launch over all members; runs of 32*dft_every steps replay a CUDA graph. */
+/* Advances every member by nsteps.  A time step is two launches
+ * over all members, an H and an E launch whose blocks are listed in device
+ * memory (line steps, dispersive cells, Yee passes), and a third at oblique
+ * incidence; runs of 32*dft_every steps replay a CUDA graph. */
 fdtd_status fdtd_batch_step(fdtd_batch* b, int nsteps, void* stream);
 /* Runs every member to Tend (fdtd_batch_step with the remaining steps). */
 fdtd_status fdtd_batch_run(fdtd_batch* b, void* stream);
@@ -488,12 +490,12 @@ fdtd_status fdtd_batch_get_stats(const fdtd_batch* b, long long* kernels,
                                  long long* graph_launches);
 /* The pass launch shapes fdtd_batch_create chose (its autotuner): members
  * are bucketed by their largest edge, 16 cells a bucket ([edge_lo, edge_hi]
- * inclusive); each bucket has its own z-chunk (planes per work item),
+ * inclusive); each bucket has its own z-chunk (planes per thread),
  * timed with the bucket's members alone (bucket_ms: both passes, one step).
- * Work items are tile_x x tile_y columns; minb / stages are the register
- * cap (minimum CTAs per SM) and ring depth of each persistent launch,
- * [0 = H pass, 1 = E pass][0 = CPML edge items, 1 = interior items], timed
- * over the whole batch.  tuned = 0 when the batch kept the defaults
+ * A warp's 32 threads take tile_x = 32 vectors of tile_y cells along x; minb
+ * / stages are the CTAs per SM and the ring depth (1 = none) of the launches,
+ * [0 = H pass, 1 = E pass], the same in both entries of the second index,
+ * timed over the whole batch.  tuned = 0 when the batch kept the defaults
  * (FDTD_TUNE=0 or under 2^20 cells). */
 #define FDTD_BATCH_MAX_BUCKETS 16
 typedef struct fdtd_batch_tuning {
