@@ -109,7 +109,7 @@ def test_unbuilt_direct_variant_is_rejected(monkeypatch):
 
 
 @pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
-@pytest.mark.parametrize("name,count", [("sphere_au", 1), ("sphere_big", 3), ("hydro", 2), ("slab", 5)])
+@pytest.mark.parametrize("name,count", [("sphere_au", 1), ("sphere_big", 3), ("hydro", 2), ("slab", 5), ("sphere_big", 9)])
 def test_batch_blocks_agree_with_single_runs(name, count, prec):
     """Batches under and over the tuner's size, members whose planes do not
     fill a block's groups, one member at oblique incidence (its TFSF launch
