@@ -1242,10 +1242,12 @@ static void update_e_comp(orc_sim* s, int c) {
           const cpml_axis* cpa = &s->cp[ax];
           int nlim = (c == 2 && ax == 1) ? Nc : Nc + 1; /* UPDATE_ez uses j<cpml_N_Y */
           if (idx_ax < nlim) {
-            const double* ceN = cpa->ce_N;
-            if (c == 1 && ax == 0 && !(s->p.fixes & FDTD_FIX_CE_EY_XN)) ceN = s->cp[1].ce_N;
+            double ceN = cpa->ce_N[idx_ax];
+            /* Ey's near-x slab takes ce_y_N (main.cu:2891), zero beyond the y slab */
+            if (c == 1 && ax == 0 && !(s->p.fixes & FDTD_FIX_CE_EY_XN))
+              ceN = idx_ax <= s->Nc[1] ? s->cp[1].ce_N[idx_ax] : 0.0;
             double* ps = &s->psiE_N[c][slot][pidx(s, ax, Nc + 1, i, j, k)];
-            *ps = cpa->be_N[idx_ax] * *ps + ceN[idx_ax] * dh / dsp[ax];
+            *ps = cpa->be_N[idx_ax] * *ps + ceN * dh / dsp[ax];
             E[id] += sg * (s->Ceh * *ps);
           }
           if (idx_ax >= s->F[ax]) {
