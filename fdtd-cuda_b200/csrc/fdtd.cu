@@ -613,6 +613,19 @@ static size_t fuse_tfsf_below(bool fp64) {
   return fp64 ? (size_t)1 << 20 : (size_t)25000000;
 }
 
+// The boxes whose corrections the passes can apply: along each axis at least 4
+// cells wide, since a thread keeps one side for the x faces in its 16-byte vector
+// (flat_faces) and a dispersive cell takes one of two opposite faces, and no face
+// on the grid's walls, whose components (and dispersive cells) the passes do not
+// store.  Other boxes keep the TFSF launch, which takes each cell by itself.
+// (Periodic x and y have no faces along those axes.)
+static bool tfsf_box_fuses(const fdtd_sim* s) {
+  const int n3[3] = {s->NX, s->NY, s->NZ};
+  for (int a = s->su.p.periodic_xy ? 2 : 0; a < 3; a++)
+    if (s->su.Nt[a] < 2 || n3[a] - 2 * s->su.Nt[a] < 4) return false;
+  return true;
+}
+
 // The direct passes (flat.cuh) run unless a knob of the staged ones is set, or
 // the grid is beyond their 32-bit cell offsets.
 static bool direct_passes(const fdtd_sim* s) {
@@ -874,7 +887,7 @@ static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out,
   // face, component and z index alone (normal incidence): the line step then
   // evaluates a few hundred increments a step.  Oblique incidence has nearly as
   // many distinct corrections as face cells and keeps the TFSF launch.
-  s->fused_tfsf = direct_passes(s.get()) && s->inc_ok && s->ncell < fuse_tfsf_below(s->fp64);
+  s->fused_tfsf = direct_passes(s.get()) && s->inc_ok && tfsf_box_fuses(s.get()) && s->ncell < fuse_tfsf_below(s->fp64);
   if (s->fused_tfsf) {
     st = s->fp64 ? fuse_tfsf<double>(s.get()) : fuse_tfsf<float>(s.get());
     if (st != FDTD_OK) return st;

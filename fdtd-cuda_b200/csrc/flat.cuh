@@ -170,8 +170,9 @@ __device__ __forceinline__ void add_lanes(Vec<T>& v, unsigned m, T x) {
 // and on which side, is fixed along a thread's planes and kept in one word:
 // bits 0-3 the x face's lane, 4-7 the y face's lanes, 8 / 9 their sides
 // (finding them per plane cost the 256^3 H pass 8 us of 121, as did keeping
-// masks and pointers apart, which spills).  The z faces are two planes of the
-// grid.  half = 0: hz, half-open in x and y; half = 1: ez, closed in x and y.
+// masks and pointers apart, which spills).  One side a vector is enough because
+// the passes take boxes of 4 cells and more only (tfsf_box_fuses, fdtd.cu).  The
+// z faces are two planes of the grid.  half = 0: hz, half-open in x and y; half = 1: ez, closed in x and y.
 template <typename T>
 __device__ __forceinline__ unsigned flat_faces(const SimView<T>& s, int half, int i0, int j) {
   constexpr int N = Vec<T>::N;
