@@ -337,6 +337,10 @@ const char* setup_build(const fdtd_params& pin, Setup& s) {
     s.scaE[a] = N3[a] - s.Nt[a] + p.box_offset;
     if (s.scaS[a] < 1 || s.scaE[a] > N3[a] - 1 || s.absE[a] - s.absS[a] < 2)
       return "TFSF/DFT boxes do not fit the grid";
+    // nor, with a box_offset below zero, may the lower TFSF faces' H cells
+    // (index Nt - 1) or the sampled absorption box lie outside it
+    if (s.Nt[a] < 1 || (p.StaticField == 0 && (s.absS[a] < 0 || s.absE[a] > N3[a])))
+      return "TFSF/DFT boxes do not fit the grid";
   }
   if (per) {
     // reflection and transmission planes (Spectral.cu:11-16)
