@@ -563,7 +563,8 @@ __global__ void metal_e(const __grid_constant__ SimView<T> s, const __grid_const
 // a == c the cells at +1, 0, -1 along c; for a != c the cells at +e_c, 0,
 // +e_c - e_a and -e_a.  cphase: components below it have already rotated
 // in this step (the reference launches UPDATE_ex, _ey, _ez in turn).
-template <typename T, int c, int cphase>
+// ny = false leaves component 1's densities to the caller.
+template <typename T, int c, int cphase, bool ny = true>
 __device__ __forceinline__ void hydro_neighbours(const MetalView<T>& m, int q, int t, double P[3][4], double N[3][4]) {
   const int* nb = m.nbr[c] + (size_t)q * 12;
 #pragma unroll
@@ -573,7 +574,7 @@ __device__ __forceinline__ void hydro_neighbours(const MetalView<T>& m, int q, i
     for (int x = 0; x < 4; x++) {
       const int sl = nb[a * 4 + x];
       P[a][x] = sl >= 0 ? m.pd[a][rp][sl] : 0.0;
-      N[a][x] = sl >= 0 ? m.nd[a][rp][sl] : 0.0;
+      if (ny || a != 1) N[a][x] = sl >= 0 ? m.nd[a][rp][sl] : 0.0;
     }
   }
 }
@@ -775,7 +776,7 @@ __device__ __forceinline__ void hydro_e_any(const SimView<T>& s, const MetalView
       }
     }
     double P[3][4], N[3][4];
-    hydro_neighbours<T, 2, 2>(m, q, t, P, N);
+    hydro_neighbours<T, 2, 2, false>(m, q, t, P, N);  // not the y cells' densities: this launch writes them
 #pragma unroll
     for (int x = 0; x < 4; x++) N[1][x] = N1[x];
     const double nd = hydro_density<T, 2>(m, t, e.w, P, N);
