@@ -504,7 +504,7 @@ static fdtd_status batch_create_impl(const fdtd_params* ps, int n, int device, f
     if (ps[i].periodic_xy) return fail(FDTD_ERR_UNSUPPORTED, "periodic_xy simulations do not batch (member " + std::to_string(i) + ")");
   for (int i = 0; i < n; i++) {
     fdtd_sim* s = nullptr;
-    const fdtd_status st = create_impl(&ps[i], device, &s, /*tune*/ false);
+    const fdtd_status st = create_impl(&ps[i], device, &s, /*member*/ true);
     if (st != FDTD_OK) return fail(st, "batch member " + std::to_string(i) + ": " + g_err);
     b->sims.emplace_back(s);
     if (i == 0) {

@@ -68,6 +68,7 @@ struct fdtd_sim {
   Setup su;
   int device = 0;
   bool fp64 = true;
+  bool member = false;  // of a batch
   int NX, NY, NZ, PX;
   size_t plane, ncell;
   int kchunk = 32;
@@ -627,15 +628,19 @@ static bool tfsf_box_fuses(const fdtd_sim* s) {
 }
 
 // The direct passes (flat.cuh) run unless a knob of the staged ones is set, or
-// the grid is beyond their 32-bit cell offsets.
+// the grid is beyond their 32-bit cell offsets.  FDTD_TMA and FDTD_PDL arrange
+// the staged launches of a simulation of its own: a batch has no such launches
+// and takes no notice of them.
 static bool direct_passes(const fdtd_sim* s) {
   const char* force = std::getenv("FDTD_PASS");
-  const bool knobs = (force && std::strncmp(force, "flat:", 5)) || std::getenv("FDTD_TMA") || std::getenv("FDTD_PDL");
+  const bool knobs = (force && std::strncmp(force, "flat:", 5)) ||
+                     (!s->member && (std::getenv("FDTD_TMA") || std::getenv("FDTD_PDL")));
   return !knobs && s->ncell < ((size_t)1 << 31);
 }
 
-static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out, bool tune = true) {
+static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out, bool member = false) {
   auto s = std::make_unique<fdtd_sim>();
+  s->member = member;
   if (const char* msg = setup_build(*p, s->su)) return fail(FDTD_ERR_INVALID, msg);
   const Setup& su = s->su;
   s->device = device;
@@ -892,7 +897,8 @@ static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out,
     st = s->fp64 ? fuse_tfsf<double>(s.get()) : fuse_tfsf<float>(s.get());
     if (st != FDTD_OK) return st;
   }
-  st = s->fp64 ? tune_passes<double>(s.get(), tune) : tune_passes<float>(s.get(), tune);
+  // (a batch times its members' passes together)
+  st = s->fp64 ? tune_passes<double>(s.get(), !member) : tune_passes<float>(s.get(), !member);
   if (st != FDTD_OK) return st;
   *out = s.release();
   return FDTD_OK;
