@@ -52,6 +52,8 @@ struct fdtd_sim::Adjoint {
   } sig;
   // adjoint state (allocated on the first backward)
   bool ready = false;
+  bool form[2] = {false, false};  // psi adjoints held: of the coefficient arrays, of the direct passes
+  bool swept_direct = false;      // the form of the reverse sweep's graph
   void* view = nullptr;  // AdjView<T> on the host, as bytes
   std::vector<char> view_bytes;
   std::vector<std::pair<void*, size_t>> zero;  // buffers zeroed before each sweep
@@ -407,6 +409,44 @@ extern "C" fdtd_status fdtd_forward(fdtd_sim* s, const int* freq_idx, int nfreq,
   return st;
 }
 
+// The transposed sub-steps as direct passes (the default; FDTD_ADJ_FUSED=0
+// selects the coefficient arrays): chh = cee = 1 and 32-bit cell offsets.
+static bool adj_direct(const fdtd_sim* s) {
+  const char* e = std::getenv("FDTD_ADJ_FUSED");
+  return s->su.Chh == 1.0 && s->su.Cee == 1.0 && s->ncell < ((size_t)1 << 31) && !(e && e[0] == '0');
+}
+
+// The psi adjoints of one form, in the shapes of the psi slabs: near and far
+// slabs apart for the coefficient arrays, together and twice for the direct
+// passes.  Only the form that runs is held.
+template <typename T>
+static fdtd_status adj_psi_alloc(fdtd_sim* s, AdjView<T>& a, bool direct) {
+  fdtd_sim::Adjoint& A = *s->adj;
+  for (int c = 0; c < 3; c++)
+    for (int slot = 0; slot < 2; slot++) {
+      const int ax = (c + 1 + slot) % 3;
+      const int Nc = s->su.Nc[ax];
+      size_t ce, ch;
+      if (ax == 2) { ce = (size_t)(Nc + 1) * s->plane; ch = (size_t)Nc * s->plane; }
+      else if (ax == 1) { ce = (size_t)s->NZ * (Nc + 1) * s->PX; ch = (size_t)s->NZ * Nc * s->PX; }
+      else { ce = (size_t)s->NZ * s->NY * (Nc + 1); ch = (size_t)s->NZ * s->NY * Nc; }
+      if (direct) {
+        const size_t row = (size_t)s->NZ * s->NY * view<T>(s).cp[0].W;
+        a.fEn[c][slot] = ax == 0 ? row : 2 * ce;
+        a.fHn[c][slot] = ax == 0 ? row : 2 * ch;
+        CUDA_TRY(A.alloc(&a.fE[c][slot], 2 * a.fEn[c][slot], true));
+        CUDA_TRY(A.alloc(&a.fH[c][slot], 2 * a.fHn[c][slot], true));
+      } else {
+        CUDA_TRY(A.alloc(&a.lpE_N[c][slot], ce, true));
+        CUDA_TRY(A.alloc(&a.lpE_F[c][slot], ce, true));
+        CUDA_TRY(A.alloc(&a.lpH_N[c][slot], ch, true));
+        CUDA_TRY(A.alloc(&a.lpH_F[c][slot], ch, true));
+      }
+    }
+  A.form[direct] = true;
+  return FDTD_OK;
+}
+
 template <typename T>
 static fdtd_status adj_prepare(fdtd_sim* s) {
   fdtd_sim::Adjoint& A = *s->adj;
@@ -425,27 +465,10 @@ static fdtd_status adj_prepare(fdtd_sim* s) {
     CUDA_TRY(A.alloc(&a.lH[c], nc, true));
     for (int q = 0; q < 2; q++) CUDA_TRY(A.alloc(&a.a[c][q], nc, false));
   }
-  // psi adjoints, the shapes of the psi slabs
   const Setup& su = s->su;
-  for (int c = 0; c < 3; c++)
-    for (int slot = 0; slot < 2; slot++) {
-      const int ax = (c + 1 + slot) % 3;
-      const int Nc = su.Nc[ax];
-      size_t ce, ch;
-      if (ax == 2) { ce = (size_t)(Nc + 1) * s->plane; ch = (size_t)Nc * s->plane; }
-      else if (ax == 1) { ce = (size_t)s->NZ * (Nc + 1) * s->PX; ch = (size_t)s->NZ * Nc * s->PX; }
-      else { ce = (size_t)s->NZ * s->NY * (Nc + 1); ch = (size_t)s->NZ * s->NY * Nc; }
-      CUDA_TRY(A.alloc(&a.lpE_N[c][slot], ce, true));
-      CUDA_TRY(A.alloc(&a.lpE_F[c][slot], ce, true));
-      CUDA_TRY(A.alloc(&a.lpH_N[c][slot], ch, true));
-      CUDA_TRY(A.alloc(&a.lpH_F[c][slot], ch, true));
-      // the direct form's: near and far together, two buffers
-      const size_t row = (size_t)s->NZ * s->NY * view<T>(s).cp[0].W;
-      a.fEn[c][slot] = ax == 0 ? row : 2 * ce;
-      a.fHn[c][slot] = ax == 0 ? row : 2 * ch;
-      CUDA_TRY(A.alloc(&a.fE[c][slot], 2 * a.fEn[c][slot], true));
-      CUDA_TRY(A.alloc(&a.fH[c][slot], 2 * a.fHn[c][slot], true));
-    }
+  A.form[0] = A.form[1] = false;
+  const fdtd_status st = adj_psi_alloc<T>(s, a, adj_direct(s));
+  if (st != FDTD_OK) return st;
   long long slots = 0;
   for (int c = 0; c < 3; c++) {
     const size_t n = std::max(1, s->nmetal[c]);
@@ -503,7 +526,17 @@ static fdtd_status adj_prepare(fdtd_sim* s) {
 template <typename T>
 static fdtd_status adj_sweep(fdtd_sim* s) {
   fdtd_sim::Adjoint& A = *s->adj;
-  const AdjView<T>& a = *reinterpret_cast<const AdjView<T>*>(A.view_bytes.data());
+  AdjView<T>& a = *reinterpret_cast<AdjView<T>*>(A.view_bytes.data());
+  const bool direct = adj_direct(s);
+  if (!A.form[direct]) {  // the other form was asked for since the forward
+    const fdtd_status st = adj_psi_alloc<T>(s, a, direct);
+    if (st != FDTD_OK) return st;
+  }
+  if (A.g_adj && A.swept_direct != direct) {
+    cudaGraphExecDestroy(A.g_adj);
+    A.g_adj = nullptr;
+  }
+  A.swept_direct = direct;
   for (const auto& z : A.zero) CUDA_TRY(cudaMemset(z.first, 0, z.second));
   MetalView<T>& m = mview<T>(s);
   adj_record_view<T>(s, true);
@@ -520,10 +553,6 @@ static fdtd_status adj_sweep(fdtd_sim* s) {
   const int nsel = (int)A.sel.size();
   const double* fsel = static_cast<const double*>(A.fsel->p) + (size_t)nsel * 12;
   const int total = A.tend + 1;
-  // the direct form (the default; FDTD_ADJ_FUSED=0 selects the coefficient
-  // arrays) needs chh = cee = 1 and 32-bit cell offsets
-  const char* fenv = std::getenv("FDTD_ADJ_FUSED");
-  const bool direct = s->su.Chh == 1.0 && s->su.Cee == 1.0 && s->ncell < ((size_t)1 << 31) && !(fenv && fenv[0] == '0');
   // planes per thread: as the forward's E pass, whose loads these are, but
   // short runs (the neighbour plane's coefficients are computed once a run)
   const int kz = std::min(std::max(s->ecfg.kz, 2), 8);
