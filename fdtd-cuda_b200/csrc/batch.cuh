@@ -178,14 +178,16 @@ struct fdtd_batch {
   }
 };
 
-// Planes per thread as blocks: a block spans 8, 16 or 32 planes (its z-chunk),
-// short runs of planes as groups of threads above one another.
-static int batch_kchunk(int kz) { return std::max(8, kz); }
+// Planes per thread as blocks: a block spans up to 8 planes, or one run where
+// that is longer (its z-chunk), short runs of planes as 2, 4 or 8 groups of
+// threads above one another.
+static int batch_groups(int kz) { return kz == 1 ? 8 : kz == 2 ? 4 : kz <= 4 ? 2 : 1; }
+static int batch_kchunk(int kz) { return kz * batch_groups(kz); }
 
 // The grid blocks of member i with kz planes per thread.
 template <typename T>
 static void batch_member_items(const fdtd_sim* s, int i, int kz, std::vector<int4>& out) {
-  const int kc = batch_kchunk(kz), groups = kc / kz, vx = kFlatThreads / groups;
+  const int kc = batch_kchunk(kz), groups = batch_groups(kz), vx = kFlatThreads / groups;
   const int nv = (int)(s->plane / Vec<T>::N), nx = (nv + vx - 1) / vx;
   for (int k = 0; k < s->NZ; k += kc)
     for (int x = 0; x < nx; x++) out.push_back(make_int4(i, x, k, kz | groups << 16));
@@ -398,6 +400,8 @@ static fdtd_status batch_time_passes(fdtd_batch* b, int reps, float* ms) {
 // alone want short runs, which fill the GPU, a full batch longer ones, which
 // re-read less.  FDTD_TUNE=0, or a batch under 2^20 cells, takes the most
 // planes, up to 8, that leave two blocks a multiprocessor.
+// FDTD_PASS=flat:KZ[:RING] fixes both (blocks have 256 threads whatever else it
+// says), FDTD_BATCH_TAIL=0 / 1 whether the last blocks are split.
 template <typename T>
 static fdtd_status batch_tune(fdtd_batch* b) {
   if (!b->direct) return FDTD_OK;
@@ -410,6 +414,15 @@ static fdtd_status batch_tune(fdtd_batch* b) {
   while (kz < 8 && vecs / (2 * kz * kFlatThreads) >= 2LL * b->sms) kz *= 2;
   for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = kz;
   const char* env = std::getenv("FDTD_TUNE");
+  const char* tail = std::getenv("FDTD_BATCH_TAIL");
+  const char* force = std::getenv("FDTD_PASS");
+  b->tail = tail && tail[0] == '1';
+  int fz = 0, fring = 0;
+  if (force && std::sscanf(force, "flat:%d:%d", &fz, &fring) >= 1) {  // (the members' creation has checked it)
+    for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = std::min(fz, 0x7FFF);
+    b->ring = fring != 0;
+    return batch_upload_items<T>(b);
+  }
   fdtd_status st;
   if ((env && env[0] == '0') || cells < (1LL << 20)) return batch_upload_items<T>(b);
   std::vector<int> chosen(b->nbuckets, kz);
@@ -440,11 +453,12 @@ static fdtd_status batch_tune(fdtd_batch* b) {
   }
   for (int q = 0; q < b->nbuckets; q++) b->bucket_kz[q] = best_z < 0 ? chosen[q] : best_z;
   b->ring = best_ring;
+  b->tuned = true;
+  if (tail) return batch_upload_items<T>(b);
   b->tail = true;
   if ((st = batch_upload_items<T>(b, -1, true)) != FDTD_OK) return st;
   if ((st = batch_time_passes<T>(b, 3, &ms)) != FDTD_OK) return st;
   b->tail = ms < best;
-  b->tuned = true;
   CUDA_TRY(cudaGetLastError());
   return batch_upload_items<T>(b);
 }
