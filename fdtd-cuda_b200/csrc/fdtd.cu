@@ -605,13 +605,17 @@ static fdtd_status fuse_tfsf(fdtd_sim* s);
 
 // Below this many cells the passes apply the TFSF corrections (FDTD_TFSF=0 / 1:
 // never / always).  In the passes they cost registers and instructions in
-// proportion to the grid, in a launch of their own a launch and the faces' cells:
-// a step with the launch against without, us, FP32 64^3 10.3 / 9.0, 96^3 20.1 /
-// 18.7, 160x144x176 72.1 / 69.3, 256^3 272 / 267, 384x384x256 563 / 568; FP64
-// (half the cells a thread) 97x89x93 27.1 / 27.0, 256^3 524 / 531.
+// proportion to the grid, in a launch of their own a launch and the faces' cells.
+// A step with the launch against without, us.  FP32 64^3 10.3 / 9.0, 96^3 20.1 /
+// 18.7, 128^3 29.8 / 30.9, 144^3 47.6 / 46.0, 160^3 62.0 / 63.3, 160x144x176
+// 72.1 / 69.3, 192^3 113 / 109, 224^3 168.8 / 170.7, 256^3 272 / 267, 384x384x256
+// 563 / 568: which wins alternates with how the blocks fill their last wave up
+// to the largest.  FP64 (half the cells a thread) 104^3 32.0 / 31.7, 112^3 44.2 /
+// 43.1, 128^3 62.9 / 59.7, 144^3 95.1 / 92.5, 160^3 125.8 / 124.8, 176^3 164.2 /
+// 167.1, 192^3 205.7 / 209.3, 208^3 261 / 270, 224^3 321 / 334, 256^3 524 / 531.
 static size_t fuse_tfsf_below(bool fp64) {
   if (const char* e = std::getenv("FDTD_TFSF")) return e[0] == '0' ? 0 : (size_t)-1;
-  return fp64 ? (size_t)1 << 20 : (size_t)25000000;
+  return fp64 ? (size_t)4700000 : (size_t)25000000;
 }
 
 // The boxes whose corrections the passes can apply: along each axis at least 4
