@@ -219,16 +219,17 @@ def cpu_sample(steps=200, grid=256, num_freq=201):
 
 def step_bytes(dims, params, st, esize):
     """Algorithmic DRAM bytes of one whole time step, by kernel family:
-    the two Yee passes (pass_bytes), the TFSF table launch (per entry: the
-    31-byte table row and a read-modify-write of one field value), the
-    dispersive cells (per component and cell: 21 state and field values
-    and the 16-byte cell entry; hydrodynamic cells add the density ring and
-    the 48-byte neighbour list), the DFT sample (a field read and a ring
-    write per row every dft_every steps) and the DFT contraction (per
-    64 samples: the ring read and a read and write of the FP64 re/im
-    accumulators of every row and frequency)."""
+    the two Yee passes (pass_bytes), the TFSF table launch where there is one
+    (per entry: the 16-byte table row and a read-modify-write of one field
+    value; none where the passes apply the corrections), the dispersive
+    cells (per component and cell: 21 state and field values and the
+    16-byte cell entry; hydrodynamic cells add the density ring and the
+    48-byte neighbour list), the DFT sample (a field read and a ring write
+    per row every dft_every steps) and the DFT contraction (per 64 samples:
+    the ring read and a read and write of the FP64 re/im accumulators of
+    every row and frequency)."""
     out = {"e_pass": pass_bytes(dims, params, esize, "e"), "h_pass": pass_bytes(dims, params, esize, "h")}
-    out["tfsf"] = (st.tfsf_entries_h + st.tfsf_entries_e) * (31 + 2 * esize)
+    out["tfsf"] = (st.tfsf_entries_h + st.tfsf_entries_e) * (16 + 2 * esize)
     nd = sum(dims.n_metal_cells)
     out["dispersive"] = nd * ((21 + (3 if dims.hydro else 0)) * esize + 16 + (48 if dims.hydro else 0))
     every = max(params.dft_every, 1)

@@ -2321,8 +2321,8 @@ extern "C" fdtd_status fdtd_get_stats(const fdtd_sim* s, fdtd_stats* out) {
   out->h_pdl = s->hcfg.pdl; out->e_pdl = s->ecfg.pdl;
   out->h_tma = s->hcfg.tma; out->h_etma = s->hcfg.etma;
   out->e_tma = s->ecfg.tma; out->e_etma = s->ecfg.etma;
-  out->tfsf_entries_h = s->tf_h.n;
-  out->tfsf_entries_e = s->tf_e.n;
+  out->tfsf_entries_h = s->fused_tfsf ? 0 : s->tf_h.n;
+  out->tfsf_entries_e = s->fused_tfsf ? 0 : s->tf_e.n;
   long long rows = 0;
   for (int f = 0; f < s->dft.nfaces; f++) rows += 4LL * s->dft.face[f].na * s->dft.face[f].nb;
   out->dft_rows = rows;

@@ -393,8 +393,9 @@ typedef struct fdtd_stats {
    * dependency, 0 = on two streams */
   int h_pdl, e_pdl;
   /* sizes of the step's work beside the passes, for traffic accounting:
-   * TFSF table entries of the H and E shells, and DFT rows (one per
-   * tangential component and flux-face cell, padding excluded) */
+   * TFSF table entries of the H and E shells (0 where the passes apply the
+   * corrections themselves), and DFT rows (one per tangential component and
+   * flux-face cell, padding excluded) */
   long long tfsf_entries_h, tfsf_entries_e, dft_rows;
   /* adjoint (after fdtd_forward / fdtd_forward_spectra): the steps whose
    * dispersive-cell trajectory the forward recorded (the backward recomputes

@@ -87,3 +87,19 @@ def batch_fields(p):
     out = [b.sim(0).field(c) for c in range(6)]
     b.close()
     return out
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+def test_statistics_tell_which_form_runs(prec, monkeypatch):
+    """The TFSF launch's entries, none where the passes apply the corrections."""
+    def entries(**over):
+        s = F.Sim(make(F, "vacuum", precision=prec, **over))
+        st = s.stats()
+        s.close()
+        return st.tfsf_entries_h, st.tfsf_entries_e
+
+    assert entries() == (0, 0)
+    for over in (dict(inc_theta_deg=20.0), BOXES[0], BOXES[6], BOXES[14], BOXES[16]):
+        assert min(entries(**over)) > 0
+    monkeypatch.setenv("FDTD_TFSF", "0")
+    assert min(entries()) > 0
