@@ -61,3 +61,35 @@ def test_form_may_change_between_sweeps(first, monkeypatch):
     for g, gp in out[1:]:
         assert np.abs(g - out[0][0]).max() <= 1e-11 * np.abs(out[0][0]).max()
         np.testing.assert_allclose(gp, out[0][1], rtol=1e-11)
+
+
+# planes per thread 2, 3, 8 (the adjoint takes 2 to 8), blocks of 128 and 256
+# threads; the last two ask the forward for the copied-ahead form and for more
+# planes than the adjoint takes
+SHAPES = ("flat:1", "flat:2", "flat:3:0:128", "flat:8:0:128", "flat:8:1", "flat:64")
+_ARRAYS = {}
+
+
+@pytest.mark.parametrize("prec", [F.FDTD_FP32, F.FDTD_FP64])
+@pytest.mark.parametrize("model", [0, 3])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_every_shape_agrees_with_the_coefficient_arrays(shape, model, prec, monkeypatch):
+    """97 x 89 x 93 cells: the same sums in the same order; the source's atomics
+    at the corners shared by two flux faces leave rounding."""
+    def gradient(mode):
+        monkeypatch.setenv("FDTD_ADJ_FUSED", mode)
+        s = design_sim(prec, Tend=300, NONLOCAL=model)
+        value = s.forward([2, 5], 40)
+        out = (value, *s.backward())
+        s.close()
+        return out
+
+    if (model, prec) not in _ARRAYS:
+        _ARRAYS[model, prec] = gradient("0")
+    value, g, gp = _ARRAYS[model, prec]
+    monkeypatch.setenv("FDTD_PASS", shape)
+    v1, g1, gp1 = gradient("1")
+    tol = 1e-11 if prec == F.FDTD_FP64 else 1e-5
+    assert v1 == value and np.abs(g).max() > 0
+    assert np.abs(g1 - g).max() <= tol * np.abs(g).max()
+    np.testing.assert_allclose(gp1, gp, rtol=tol)
