@@ -8,9 +8,9 @@
 //
 // The transposed Yee/CPML sub-steps are written in gather form and run as the
 // direct passes of adj_flat.cuh; the form they must agree with (and the one for
-// grids beyond 32-bit offsets) stands here: a first kernel turns each updated component's adjoint into the coefficients of
-// the field differences it read ("a" arrays, one per component and
-// difference axis) and applies the psi recursions transposed; a second
+// grids beyond 32-bit offsets) stands here: a first kernel turns each updated
+// component's adjoint into the coefficients of the field differences it read
+// ("a" arrays, one per component and difference axis) and applies the psi recursions transposed; a second
 // kernel gathers those coefficients into the adjoint of the other field
 // (each difference D = F(p) - F(p - e) read by cell p contributes +a(p) to
 // F(p) and -a(p) to F(p - e)).  The dispersive (design) cells transpose
@@ -229,12 +229,12 @@ __global__ void adj_e_design(const __grid_constant__ SimView<T> s, const __grid_
 }
 
 // ---------------------------------------------------------------------
-// Hydrodynamic cells, transposed.  The forward step (kernels.cuh) is three
-// phases: hydro_p_any computes J^{n+1} of every cell from J^n, J^{n-1},
-// E^n, E^{n-1} and the pressure term over the neighbour slots' J^n and
-// N^n, then the x cells' continuity and E update; hydro_e<1> and <2> do the
-// y and z cells, whose continuity reads the x (and y) neighbours' new J and
-// N.  Linearised about the recorded trajectory (MetalView::hrec, ::rec),
+// Hydrodynamic cells, transposed.  The forward step (kernels.cuh) has two
+// parts: hydro_p_any computes J^{n+1} of every cell from J^n, J^{n-1}, E^n,
+// E^{n-1} and the pressure term over the neighbour slots' J^n and N^n, and the
+// x cells' new density; hydro_e_any computes the y and z cells' densities,
+// whose continuity reads the x (and y) neighbours' new J and N (a z cell
+// computes its y neighbours' again), and every E.  Linearised about the recorded trajectory (MetalView::hrec, ::rec),
 // the reverse step runs adj_hydro_e<2>, <1>, <0> (E update and continuity
 // of each phase, in reverse order), then adj_hydro_j (the current update).
 // A slot's J or N adjoint receives terms from its neighbours, added with

@@ -50,7 +50,7 @@ struct fdtd_sim::Adjoint {
     const void* fsel = nullptr;
     bool operator==(const ObjSig& o) const { return nsel == o.nsel && mask == o.mask && P == o.P && fsel == o.fsel; }
   } sig;
-  // adjoint state (allocated on the first backward)
+  // adjoint state (allocated by the forward)
   bool ready = false;
   bool form[2] = {false, false};  // psi adjoints held: of the coefficient arrays, of the direct passes
   bool swept_direct = false;      // the form of the reverse sweep's graph

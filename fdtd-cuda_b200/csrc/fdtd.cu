@@ -73,9 +73,8 @@ struct fdtd_sim {
   size_t plane, ncell;
   int kchunk = 32;
   // launch shape of the E and H passes, chosen by tune_passes()
-  // staged = shared-memory pipelined kernels (minb unused), else the plain
-  // register z-march
-  // launch shape of one pass: tile height and z-chunk shared by its two
+  // staged = shared-memory pipelined kernels, else the direct passes
+  // launch shape of one staged pass: tile height and z-chunk shared by its two
   // launches, register cap (min CTAs/SM) and ring depth per launch
   // (interior tiles: minb/stages, CPML edge tiles: eminb/estages)
   // pdl = 1: the edge and interior launches of a pass go on one stream
@@ -1291,17 +1290,13 @@ static int launch_e_cfg(fdtd_sim* s, const fdtd_sim::PassCfg& c, cudaStream_t st
   return launch_pass_cfg<T, true>(s, c, st, chained);
 }
 
-// Autotuner of the staged passes: times every launch shape of the E and H passes on the zero
-// state (which they leave at zero: no source has run yet) and keeps the
-// fastest.  Shapes: minimum CTAs per SM (register cap) x tile height x
-// z-chunk.  FDTD_TUNE=0 keeps the defaults.
-
-// The direct passes: planes per thread of each pass, and whether they are copied
-// ahead.  More planes per thread re-read less (the k +- 1 plane is carried) but
-// leave fewer blocks, so small grids want few and wave quantisation decides in
-// between: timed on the zero state like the staged shapes.  Untimed (FDTD_TUNE=0,
-// batch members, under 2^18 cells) the most planes, up to 8, that leave two
-// blocks a multiprocessor, copied ahead from 4 planes on.
+// Autotuner of the direct passes: planes per thread of each pass, threads per
+// block, and whether the planes are copied ahead.  More planes per thread re-read
+// less (the k +- 1 plane is carried) but leave fewer blocks, so small grids want
+// few and wave quantisation decides in between: timed as graphs of launches on the
+// zero state (which they leave at zero: no source has run yet).  Untimed
+// (FDTD_TUNE=0, batch members, under 2^18 cells) the most planes, up to 8, that
+// leave two blocks a multiprocessor, copied ahead from 4 planes on.
 // FDTD_PASS=flat:KZ[:RING[:THREADS]] fixes them.
 template <typename T>
 static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force) {
@@ -1415,6 +1410,10 @@ static fdtd_status tune_flat(fdtd_sim* s, bool time_variants, const char* force)
   return FDTD_OK;
 }
 
+// Sets the launch shapes of the E and H passes: the direct passes' above, or, for
+// the staged ones, the fastest of every shape timed on the zero state: minimum
+// CTAs per SM (register cap) x tile height x z-chunk.  FDTD_TUNE=0 keeps the
+// defaults.
 template <typename T>
 static fdtd_status tune_passes(fdtd_sim* s, bool time_variants) {
   CUDA_TRY(cudaFuncSetAttribute(dft_contract<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_smem_bytes<T>()));
@@ -1731,15 +1730,16 @@ static void launch_snap(fdtd_sim* s, cudaStream_t st) {
   s->kernels++;
 }
 
-// One full step.  The 1-D line step runs beside the H pass (on the second
-// side stream, or before it on the same stream with the pass launched as a
-// programmatic dependent when the pass's launches run on one stream): it
-// reads the line, E at the probe cell and the clock, none of which the H
-// pass touches, and writes the line's other E buffer, so the H half of
-// CORRECT_* still sees the line's E from before the update, as in the
-// reference's order (UPDATE_h*, CORRECT_* H, UPDATE_h_inc/e_inc, CORRECT_* E,
-// UPDATE_e*).  Both TFSF halves then run as one launch.  Host
-// mirrors of the clock decide which optional kernels run; the kernels read
+// One full step.  The 1-D line step runs beside the H pass (the direct passes:
+// a block of the same launch; the staged ones: on the second side stream, or
+// before the pass on the same stream with the pass launched as a programmatic
+// dependent when its launches run on one stream).  It reads the line, E at the
+// probe cell and the clock, none of which the H pass touches, and writes the
+// line's other E buffer, so the H half of CORRECT_* still sees the line's E
+// from before the update, as in the reference's order (UPDATE_h*, CORRECT_* H,
+// UPDATE_h_inc/e_inc, CORRECT_* E, UPDATE_e*).  The passes add the corrections
+// themselves (fused_tfsf), or both TFSF halves run as one launch after the line.
+// Host mirrors of the clock decide which optional kernels run; the kernels read
 // t from the device.
 template <typename T>
 static void enqueue_step(fdtd_sim* s, cudaStream_t st) {

@@ -34,7 +34,7 @@ __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
 // multiply-adds that the compiler may neither contract nor split.  The Yee
 // passes are written with these, so that a cell's update rounds the same
 // in every launch form (the CPML-free or the CPML-edge instantiation, any
-// tile shape, the batched work queue).
+// tile shape, the batch).
 __device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }

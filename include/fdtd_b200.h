@@ -390,7 +390,7 @@ typedef struct fdtd_stats {
   /* the same two for the staged launch over the CPML edge tiles */
   int h_eminb, h_estages, e_eminb, e_estages;
   /* 1 = the two launches of the pass run on one stream with a programmatic
-   * dependency, 0 = on two streams */
+   * dependency, 0 = on two streams (direct passes, one launch: 1) */
   int h_pdl, e_pdl;
   /* sizes of the step's work beside the passes, for traffic accounting:
    * TFSF table entries of the H and E shells (0 where the passes apply the
@@ -491,13 +491,13 @@ fdtd_status fdtd_batch_get_stats(const fdtd_batch* b, long long* kernels,
                                  long long* graph_launches);
 /* The pass launch shapes fdtd_batch_create chose (its autotuner): members
  * are bucketed by their largest edge, 16 cells a bucket ([edge_lo, edge_hi]
- * inclusive); each bucket has its own z-chunk (planes per thread),
- * timed with the bucket's members alone (bucket_ms: both passes, one step).
+ * inclusive); each bucket has its own z-chunk (the planes a block spans:
+ * a thread's, or 2, 4 or 8 short runs of planes above one another), timed with the bucket's members alone (bucket_ms: both passes, one step).
  * A warp's 32 threads take tile_x = 32 vectors of tile_y cells along x; minb
  * / stages are the CTAs per SM and the ring depth (1 = none) of the launches,
  * [0 = H pass, 1 = E pass], the same in both entries of the second index,
  * timed over the whole batch.  tuned = 0 when the batch kept the defaults
- * (FDTD_TUNE=0 or under 2^20 cells). */
+ * (FDTD_TUNE=0 or under 2^20 cells) or FDTD_PASS=flat fixed them. */
 #define FDTD_BATCH_MAX_BUCKETS 16
 typedef struct fdtd_batch_tuning {
   int tuned;
