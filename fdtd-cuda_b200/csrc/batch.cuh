@@ -10,6 +10,8 @@
 //   h_flat_batch      line steps, hydrodynamic currents, H pass
 //   tfsf_apply_batch  only with members at oblique incidence
 //   e_flat_batch      dispersive cells, E pass
+//   metal_e_batch, hydro_p_batch, hydro_e_batch  the dispersive cells beside the
+//                     E pass where they are many (cells_apart, fdtd.cu)
 //   dft_sample        one launch every dft_every steps, blockIdx.z = member
 //   the DFT contraction (job, phasors, product, reset), one launch each,
 //                     every 32 samples; it contracts each member's first
@@ -102,6 +104,21 @@ __global__ void __launch_bounds__(kFlatThreads, 2)
   e_flat_cells<T, RING, true>(s, (unsigned)(it.y * vx + (threadIdx.x - tz * vx)), it.z + tz * kz, kz);
 }
 template <typename T>
+__global__ void metal_e_batch(const BatchSim<T>* __restrict__ b) {
+  const BatchSim<T>& x = b[blockIdx.y];
+  metal_e_cell(x.v, x.m, x.clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+}
+template <typename T>
+__global__ void hydro_p_batch(const BatchSim<T>* __restrict__ b) {
+  const BatchSim<T>& x = b[blockIdx.y];
+  hydro_p_any(x.v, x.m, x.clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+}
+template <typename T, int PART>
+__global__ void hydro_e_batch(const BatchSim<T>* __restrict__ b) {
+  const BatchSim<T>& x = b[blockIdx.y];
+  hydro_e_part<T, PART>(x.v, x.m, x.clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+}
+template <typename T>
 __global__ void dft_sample_batch(const BatchSim<T>* __restrict__ b) {
   const BatchSim<T>& x = b[blockIdx.z];
   dft_sample_body(x.v, x.dft, x.ring, x.clk);
@@ -157,6 +174,10 @@ struct fdtd_batch {
   std::vector<int> member_bucket;
   int sms = 0;
   bool tuned = false;
+  bool cells_apart = false;  // the dispersive cells run as launches of their own
+  unsigned g_m = 0;          // their blocks of 128 (the largest member's)
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   unsigned g_f = 0, g_s = 0, g_tw = 0, g_c = 0;
   int t = 0, host_nsamp = 0, dft_every = 0, tend = 0;
   long long kernels = 0, graph_launches = 0, graph_kernels = 0;
@@ -166,6 +187,9 @@ struct fdtd_batch {
   ~fdtd_batch() {
     if (graph) cudaGraphExecDestroy(graph);
     if (cap) cudaStreamDestroy(cap);
+    if (side) cudaStreamDestroy(side);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
   }
   template <typename U>
   cudaError_t alloc(U** out, size_t count) {
@@ -197,6 +221,7 @@ template <typename T>
 static fdtd_status batch_build(fdtd_batch* b) {
   const int n = (int)b->sims.size();
   std::vector<BatchSim<T>> d(n);
+  long long cells = 0;
   for (int i = 0; i < n; i++) {
     fdtd_sim* s = b->sims[i].get();
     BatchSim<T>& x = d[i];
@@ -214,6 +239,9 @@ static fdtd_status batch_build(fdtd_batch* b) {
     x.clk = s->clk;
     x.probe_id = s->probe_id;
     auto blocks = [](long long cells, int per) { return (unsigned)((cells + per - 1) / per); };
+    const long long nc = (long long)s->nmetal[0] + s->nmetal[1] + s->nmetal[2];
+    cells += nc;
+    b->g_m = std::max(b->g_m, blocks(nc, 128));
     b->g_f = std::max(b->g_f, blocks((long long)x.tf_h.n + x.tf_e.n, 256));
     int maxn = 0;
     for (int f = 0; f < 12; f++) maxn = std::max(maxn, s->dft.face[f].na * s->dft.face[f].nb);
@@ -251,6 +279,12 @@ static fdtd_status batch_build(fdtd_batch* b) {
     b->bucket_members[q]++;
   }
   CUDA_TRY(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
+  b->cells_apart = cells_apart(cells, b->sms, 8);
+  if (b->cells_apart) {
+    CUDA_TRY(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+    CUDA_TRY(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+  }
   {
     const void* k[4] = {(const void*)h_flat_batch<T, true, false>, (const void*)h_flat_batch<T, true, true>,
                         (const void*)e_flat_batch<T, true, false>, (const void*)e_flat_batch<T, true, true>};
@@ -292,7 +326,7 @@ static fdtd_status batch_upload_items(fdtd_batch* b, int only = -1, bool grid = 
     std::vector<int4> v;
     if (!grid && p == 0)
       for (int i = 0; i < n; i++) v.push_back(make_int4(i | kItemLine << 20, 0, 0, 0));
-    if (!grid && (p == 1 || b->hydro))
+    if (!grid && !b->cells_apart && (p == 1 || b->hydro))
       for (int i = 0; i < n; i++) {
         const fdtd_sim* s = b->sims[i].get();
         const int nb = (s->nmetal[0] + s->nmetal[1] + s->nmetal[2] + kFlatThreads - 1) / kFlatThreads;
@@ -350,7 +384,23 @@ static void batch_enqueue_step(fdtd_batch* b, cudaStream_t st) {
   int k = 2;
   batch_launch<T>(b, 0, st);
   if (b->g_f) { tfsf_apply_batch<T><<<dim3(b->g_f, n), 256, 0, st>>>(d); k++; }
+  if (b->cells_apart) {
+    const dim3 g(b->g_m, n);
+    cudaEventRecord(b->fork, st);
+    cudaStreamWaitEvent(b->side, b->fork, 0);
+    if (!b->hydro) {
+      metal_e_batch<T><<<g, 128, 0, b->side>>>(d);
+      k++;
+    } else {
+      hydro_p_batch<T><<<g, 128, 0, b->side>>>(d);
+      hydro_e_batch<T, 1><<<g, 128, 0, b->side>>>(d);
+      hydro_e_batch<T, 2><<<g, 128, 0, b->side>>>(d);
+      k += 3;
+    }
+    cudaEventRecord(b->join, b->side);
+  }
   batch_launch<T>(b, 1, st);
+  if (b->cells_apart) cudaStreamWaitEvent(st, b->join, 0);
   if (b->dft_every > 0 && b->t % b->dft_every == 0) {
     dft_sample_batch<T><<<dim3(b->g_s, 12, n), 256, 0, st>>>(d);
     k++;

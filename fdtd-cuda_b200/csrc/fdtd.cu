@@ -69,6 +69,7 @@ struct fdtd_sim {
   int device = 0;
   bool fp64 = true;
   bool member = false;  // of a batch
+  bool cells_apart = false;  // the dispersive cells run as launches of their own
   int NX, NY, NZ, PX;
   size_t plane, ncell;
   int kchunk = 32;
@@ -599,6 +600,22 @@ static fdtd_status build_tfsf_table(fdtd_sim* s, const ShellCells& sh, int efiel
   return FDTD_OK;
 }
 
+// Dispersive cells run in blocks of the pass launches (128 registers, 16 warps a
+// multiprocessor, in front of the grid's blocks) up to one wave of those blocks,
+// and beyond it in launches of their own beside the E pass (72 to 88 registers).
+// Blocks against launches, a step in us: local model FP32 64^3 with 49,000 cells
+// 11.6 / 11.8, 73,000 11.9 / 11.9, 128^3 with 116,000 39.7 / 34.6, 930,000
+// 86.1 / 69.4, 4.2 million 292 / 194; hydrodynamic 64^3 73,000 16.1 / 19.2, 128^3
+// 116,000 47.8 / 43.5, 1.6 million 227 / 147; FP64 128^3 116,000 70.2 / 69.0,
+// 4.2 million 308 / 255.  A batch's blocks have more beside them: from 8 waves on,
+// 64 members with 369,000 cells 1026 / 1030, 8 with 1.4 million 231 / 219, 6
+// hydrodynamic ones with 752,000 193 / 159.  FDTD_CELLS=0 / 1: blocks / launches
+// whatever the count.
+static bool cells_apart(long long cells, int sms, int waves = 1) {
+  if (const char* e = std::getenv("FDTD_CELLS")) return cells > 0 && e[0] == '1';
+  return cells > 2LL * sms * kFlatThreads * waves;
+}
+
 template <typename T>
 static fdtd_status fuse_tfsf(fdtd_sim* s);
 
@@ -900,6 +917,9 @@ static fdtd_status create_impl(const fdtd_params* p, int device, fdtd_sim** out,
     st = s->fp64 ? fuse_tfsf<double>(s.get()) : fuse_tfsf<float>(s.get());
     if (st != FDTD_OK) return st;
   }
+  int sms = 148;
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  s->cells_apart = cells_apart((long long)s->nmetal[0] + s->nmetal[1] + s->nmetal[2], sms);
   // (a batch times its members' passes together)
   st = s->fp64 ? tune_passes<double>(s.get(), !member) : tune_passes<float>(s.get(), !member);
   if (st != FDTD_OK) return st;
@@ -1602,7 +1622,7 @@ static void launch_e(fdtd_sim* s, cudaStream_t st) {
     tfsf_e_apply<T><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(view<T>(s), s->tf_e);
     s->kernels++;
   }
-  if (s->ecfg.kz) {
+  if (s->ecfg.kz && !s->cells_apart) {
     // the fused step computes the hydrodynamic currents in its H launch
     const int ntot = s->nmetal[0] + s->nmetal[1] + s->nmetal[2];
     if (s->su.hydro && ntot > 0) {
@@ -1633,8 +1653,10 @@ static void launch_e_pass(fdtd_sim* s, cudaStream_t st) {
   // the E pass: the pass skips them, reads no dispersive E component and
   // writes none, and the dispersive kernels read E^n of their own cells and
   // the final H only.
+  // (The direct passes' blocks of the first waves leave the cells' launch its
+  // room: in line before the pass it measured 1 to 15% slower a step.)
   const bool metal = s->nmetal[0] + s->nmetal[1] + s->nmetal[2] > 0;
-  if (metal && s->ecfg.pdl) {
+  if (metal && s->ecfg.pdl && !s->ecfg.kz) {
     // one stream, without a fork: the dispersive kernels, then the pass,
     // each launch with a programmatic dependency on the one before (a
     // dispersive phase waits for the previous phase at its start, the pass
@@ -1655,9 +1677,9 @@ static void launch_e_pass(fdtd_sim* s, cudaStream_t st) {
   }
 }
 
-// The dispersive cells' kernels (staged passes); chained: the hydrodynamic E
-// update carries a programmatic dependency on the currents' launch (it waits
-// for it at its start).
+// The dispersive cells' launches; chained: the hydrodynamic E updates carry a
+// programmatic dependency on the launch before (they wait for it at their
+// start).
 template <typename T>
 static void launch_metal(fdtd_sim* s, cudaStream_t st, bool chained) {
   const int ntot = s->nmetal[0] + s->nmetal[1] + s->nmetal[2];
@@ -1668,9 +1690,17 @@ static void launch_metal(fdtd_sim* s, cudaStream_t st, bool chained) {
   } else {
     // UpdateHydroP* of every cell, then the E updates
     hydro_p<T><<<(ntot + 127) / 128, 128, 0, st>>>(view<T>(s), mview<T>(s), s->clk);
-    launch_ex(chained, hydro_e<T>, dim3((ntot + 127) / 128), dim3(128), 0, st, view<T>(s), mview<T>(s),
-              (const DevClock*)s->clk);
-    s->kernels += 2;
+    s->kernels++;
+    auto part = [&](void (*k)(SimView<T>, MetalView<T>, const DevClock*), int n) {
+      if (n == 0) return;
+      launch_ex(chained, k, dim3((n + 127) / 128), dim3(128), 0, st, view<T>(s), mview<T>(s), (const DevClock*)s->clk);
+      s->kernels++;
+    };
+    if (!s->cells_apart) part(hydro_e<T, 0>, ntot);
+    else {
+      part(hydro_e<T, 1>, s->nmetal[0] + s->nmetal[1]);
+      part(hydro_e<T, 2>, s->nmetal[2]);
+    }
   }
 }
 template <typename T>
@@ -1746,15 +1776,20 @@ static void enqueue_step(fdtd_sim* s, cudaStream_t st) {
   dft_period_begin<T>(s, st);
   if (s->hcfg.kz) {
     // two launches a step: H with the line and the hydrodynamic currents, E with
-    // the dispersive cells (and the TFSF launch between them where the passes do
+    // the dispersive cells where these are few (and the TFSF launch between them where the passes do
     // not apply it).  Plain launches: with programmatic dependencies the next
     // launch's blocks, resident early, take the slots that free first and the
     // single-wave passes end up unevenly spread (97 x 89 x 93 FP64 33.0 us a step
     // against 26.5, 96^3 20.8 against 18.3, 256^3 FP32 250.3 against 246.2).
-    launch_flat<T, false>(s, s->hcfg, st, true, true);
+    launch_flat<T, false>(s, s->hcfg, st, true, !s->cells_apart);
     launch_tfsf<T>(s, st);
-    launch_flat<T, true>(s, s->ecfg, st, false, true);
-    s->kernels += 2;
+    s->kernels++;
+    if (s->cells_apart) {
+      launch_e_pass<T>(s, st);
+    } else {
+      launch_flat<T, true>(s, s->ecfg, st, false, true);
+      s->kernels++;
+    }
     if (s->line.dft_every > 0 && s->t % s->line.dft_every == 0) sample_and_contract<T>(s, st);
     if (s->snap_on) launch_snap<T>(s, st);
     s->t++;

@@ -740,6 +740,36 @@ __device__ __forceinline__ void hydro_p_any(const SimView<T>& s, const MetalView
   else if (c == 1) hydro_p_cell<T, 1>(s, m, t, q);
   else if (c == 2) hydro_p_cell<T, 2>(s, m, t, q);
 }
+// E of z cell q.  OWN: computes its neighbours' new y densities itself, else
+// they are there.
+template <typename T, bool OWN>
+__device__ __forceinline__ void hydro_z_cell(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
+  const int rnew = (t + 1) % 3;
+  const int4 e = m.cell[2][q];
+  double N1[4];
+  if (OWN) {
+    const int* nb = m.nbr[2] + (size_t)q * 12 + 4;
+#pragma unroll 1
+    for (int x = 0; x < 4; x++) {
+      const int sl = nb[x];
+      N1[x] = 0.0;
+      if (sl >= 0) {
+        double P[3][4], N[3][4];
+        hydro_neighbours<T, 1, 1>(m, sl, t, P, N);  // a cell's list entry is its slot
+        N1[x] = hydro_density<T, 1>(m, t, sl, P, N);
+      }
+    }
+  }
+  double P[3][4], N[3][4];
+  hydro_neighbours<T, 2, 2, !OWN>(m, q, t, P, N);  // OWN: not the y cells' densities, which this launch writes
+  if (OWN) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) N[1][x] = N1[x];
+  }
+  const double nd = hydro_density<T, 2>(m, t, e.w, P, N);
+  m.nd[2][rnew][e.w] = nd;
+  hydro_e_cell<T, 2>(s, m, t, e, nd, m.pd[2][rnew][e.w]);
+}
 // E of one cell once every new current and every new x density are there: an
 // x cell reads its density, a y cell computes its own from neighbours that are
 // all new, a z cell needs the new y densities of up to four neighbours and
@@ -762,42 +792,35 @@ __device__ __forceinline__ void hydro_e_any(const SimView<T>& s, const MetalView
     m.nd[1][rnew][e.w] = nd;
     hydro_e_cell<T, 1>(s, m, t, e, nd, m.pd[1][rnew][e.w]);
   } else {
-    const int4 e = m.cell[2][q];
-    double N1[4];
-    const int* nb = m.nbr[2] + (size_t)q * 12 + 4;
-#pragma unroll 1
-    for (int x = 0; x < 4; x++) {
-      const int sl = nb[x];
-      N1[x] = 0.0;
-      if (sl >= 0) {
-        double P[3][4], N[3][4];
-        hydro_neighbours<T, 1, 1>(m, sl, t, P, N);  // a cell's list entry is its slot
-        N1[x] = hydro_density<T, 1>(m, t, sl, P, N);
-      }
-    }
-    double P[3][4], N[3][4];
-    hydro_neighbours<T, 2, 2, false>(m, q, t, P, N);  // not the y cells' densities: this launch writes them
-#pragma unroll
-    for (int x = 0; x < 4; x++) N[1][x] = N1[x];
-    const double nd = hydro_density<T, 2>(m, t, e.w, P, N);
-    m.nd[2][rnew][e.w] = nd;
-    hydro_e_cell<T, 2>(s, m, t, e, nd, m.pd[2][rnew][e.w]);
+    hydro_z_cell<T, true>(s, m, t, q);
+  }
+}
+// Part of the E updates as a launch: 0 = all, 1 = the x and y cells, 2 = the z
+// cells after them.
+template <typename T, int PART>
+__device__ __forceinline__ void hydro_e_part(const SimView<T>& s, const MetalView<T>& m, int t, int q) {
+  if (PART == 2) {
+    if (q < m.n[2]) hydro_z_cell<T, false>(s, m, t, q);
+  } else if (PART == 0 || q < m.n[0] + m.n[1]) {
+    hydro_e_any(s, m, t, q);
   }
 }
 
-// The hydrodynamic step as two launches of its own: the currents, then E.
+// The hydrodynamic step as launches of its own: the currents, then E, at once or
+// (many cells: the densities that z cells compute again cost more than a launch)
+// the z cells after the others.
 template <typename T>
 __global__ void hydro_p(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
                         const DevClock* clk) {
   pdl_launch_dependents();  // the next launch waits for this one itself; the E pass touches none of its cells
   hydro_p_any(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
 }
-template <typename T>
+template <typename T, int PART>
 __global__ void hydro_e(const __grid_constant__ SimView<T> s, const __grid_constant__ MetalView<T> m,
                         const DevClock* clk) {
   pdl_launch_dependents();
-  pdl_wait();  // the currents are there
-  hydro_e_any(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
+  pdl_wait();  // the launch before has finished
+  hydro_e_part<T, PART>(s, m, clk->t - 1, (int)(blockIdx.x * blockDim.x + threadIdx.x));
 }
 
 // ---------------------------------------------------------------------
