@@ -28,7 +28,9 @@
 //
 // The line, the dispersive cells and the TFSF increments ride in the two
 // launches: a step in seven launches on side streams was 13.5 us at 64^3 and
-// 292 us for the 256^3 dimer with these passes, in two 9.1 and 267.
+// 292 us for the 256^3 dimer with these passes, in two 9.1 and 267.  (Beyond one
+// wave of blocks the dispersive cells have launches of their own: cells_apart,
+// fdtd.cu.)
 #pragma once
 #include "kernels.cuh"
 

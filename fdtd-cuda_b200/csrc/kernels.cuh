@@ -10,6 +10,8 @@
 //   e_flat      the dispersive cells' E updates (Drude + 2CP, hydrodynamic;
 //               compact lists) and UPDATE_ex/ey/ez for the other
 //               components + E CPML
+//   metal_e, or hydro_p and hydro_e, beside e_flat where the dispersive cells
+//               are many, in place of their blocks in the two launches
 // and beside them
 //   dft_sample  every dft_every steps: gather the flux-plane tangential
 //               components into a sample ring
